@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(kInvThreads) block_inverse_kernel(const double
             }
         __syncthreads();
         const double rp = 1.0 / sA[k * n + k];
+        __syncthreads();  // every thread has read the pivot before its entry is scaled
         // scale row k (its pivot entry becomes 1/a_kk); keep column k's multipliers
         for (int j = tid; j < n; j += kInvThreads) sA[j * n + k] = (j == k ? 1.0 : sA[j * n + k]) * rp;
         for (int i = tid; i < n; i += kInvThreads) fcol[i] = sA[k * n + i];
