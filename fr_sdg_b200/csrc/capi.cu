@@ -37,6 +37,9 @@ FRSDG_DECL_ALL(cplx)
 #define FRSDG_DECL2(S, N) extern template cudaError_t launch_fr2d<S, N>(int, int, int, const Fr2dArgs&, cudaStream_t);
 FRSDG_DECL2(float, 2) FRSDG_DECL2(float, 3) FRSDG_DECL2(float, 4) FRSDG_DECL2(float, 5) FRSDG_DECL2(float, 6)
 FRSDG_DECL2(float, 7) FRSDG_DECL2(float, 8) FRSDG_DECL2(float, 9) FRSDG_DECL2(float, 10)
+#define FRSDG_DECLJ(N) extern template cudaError_t launch_jac2d<N>(int, int, const Fr2dArgs&, const JacOut&, cudaStream_t);
+FRSDG_DECLJ(2) FRSDG_DECLJ(3) FRSDG_DECLJ(4) FRSDG_DECLJ(5) FRSDG_DECLJ(6) FRSDG_DECLJ(7) FRSDG_DECLJ(8) FRSDG_DECLJ(9)
+FRSDG_DECLJ(10)
 } // namespace frsdg
 
 namespace
@@ -69,6 +72,22 @@ template <class S> cudaError_t dispatch2d(int n, int gas, int riem, int geo, con
         case 8: return launch_fr2d<S, 8>(gas, riem, geo, a, s);
         case 9: return launch_fr2d<S, 9>(gas, riem, geo, a, s);
         case 10: return launch_fr2d<S, 10>(gas, riem, geo, a, s);
+        default: return cudaErrorInvalidValue;
+    }
+}
+cudaError_t dispatch_jac2d(int n, int gas, int riem, const Fr2dArgs& a, const JacOut& o, cudaStream_t s)
+{
+    switch (n)
+    {
+        case 2: return launch_jac2d<2>(gas, riem, a, o, s);
+        case 3: return launch_jac2d<3>(gas, riem, a, o, s);
+        case 4: return launch_jac2d<4>(gas, riem, a, o, s);
+        case 5: return launch_jac2d<5>(gas, riem, a, o, s);
+        case 6: return launch_jac2d<6>(gas, riem, a, o, s);
+        case 7: return launch_jac2d<7>(gas, riem, a, o, s);
+        case 8: return launch_jac2d<8>(gas, riem, a, o, s);
+        case 9: return launch_jac2d<9>(gas, riem, a, o, s);
+        case 10: return launch_jac2d<10>(gas, riem, a, o, s);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -156,10 +175,8 @@ static void free_handle(frsdg_handle* h)
     cudaFree(h->d_work);
     cudaFree(h->d_stage);
     cudaFree(h->d_bad);
-    cudaFree(h->d_blocks);
     cudaFree(h->d_inv);
     cudaFree(h->d_singular);
-    cudaFree(h->d_blocks5);
     cudaFree(h->d_off);
     for (cudaStream_t& q : h->hst)
         if (q) cudaStreamDestroy(q);
@@ -337,7 +354,6 @@ int frsdg_create(const frsdg_config* cfg, frsdg_handle** out)
         a.nd = 4 * n * n;
         a.exact_bc = cfg->jvp_exact_bc;
         a.tc = cfg->mixed_tc ? 1 : 0;
-        a.jac_cmode = ((per_x && (Nx & 1)) || (per_y && (Ny & 1))) ? 1 : 0;
         for (int d = 0; d < 4; ++d)
         {
             a.bc[d].kind = cfg->bc[d].kind;
@@ -784,60 +800,31 @@ int frsdg_set_row_window(frsdg_handle* h, int row_base, int rows, int row_begin,
     return FRSDG_OK;
 }
 
+// Checks and launch of the Jacobian's element blocks (jac2d.cuh).
+static int run_jac(frsdg_handle* h, double t, double sigma, const double* U, const JacOut& o, void* stream)
+{
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    h->last = s;
+    Fr2dArgs a = h->a2;
+    a.t = t;
+    a.cond_sys = h->cfg.cond_sys;
+    a.U = U;
+    a.h = h->cfg.csd_eps;
+    a.inv_h = 1.0 / h->cfg.csd_eps;
+    a.sigma = sigma;
+    apply_window(h, a);
+    const cudaError_t e = dispatch_jac2d(h->n, h->cfg.gas_law, h->cfg.riemann, a, o, s);
+    if (e != cudaSuccess) return cuda_fail(e, "Jacobian-block launch");
+    return FRSDG_OK;
+}
+
 int frsdg_jac_blocks(frsdg_handle* h, double t, double sigma, const double* U, double* blocks, void* stream)
 {
     if (!h || !U || !blocks) return fail(FRSDG_ERR_ARG, "null argument");
     if (h->cfg.dim != 2) return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_jac_blocks: 2D configurations only");
     if ((reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(blocks)) & 15)
         return fail(FRSDG_ERR_ARG, "device pointers must be 16-byte aligned");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    h->last = s;
-    Fr2dArgs a = h->a2;
-    a.t = t;
-    a.mode = MODE_JAC;
-    a.cond_sys = h->cfg.cond_sys;
-    a.U = U;
-    a.W = nullptr;
-    a.out = blocks;
-    a.h = h->cfg.csd_eps;
-    a.inv_h = 1.0 / h->cfg.csd_eps;
-    a.sigma = sigma;
-    apply_window(h, a);
-    const cudaError_t e = dispatch2d<cplx>(h->n, h->cfg.gas_law, h->cfg.riemann, h->geo, a, s);
-    if (e != cudaSuccess) return cuda_fail(e, "Jacobian-block launch");
-    return FRSDG_OK;
-}
-
-int frsdg_pc_setup(frsdg_handle* h, double t, double sigma, const double* U, void* stream)
-{
-    if (!h || !U) return fail(FRSDG_ERR_ARG, "null argument");
-    if (h->cfg.dim != 2) return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_setup: 2D configurations only");
-    const int nd = h->ndofs;
-    if (nd > kMaxBlockDofs) return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_setup: element blocks above 144 DOFs (p > 5)");
-    cudaError_t e;
-    if (!h->d_blocks)
-    {
-        const size_t nb = size_t(h->nelem) * nd * nd;
-        if ((e = cudaMalloc(&h->d_blocks, sizeof(double) * nb)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(blocks)");
-        if ((e = cudaMalloc(&h->d_inv, sizeof(float) * nb)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(inverse blocks)");
-        if ((e = cudaMalloc(&h->d_singular, sizeof(unsigned long long))) != cudaSuccess)
-            return cuda_fail(e, "cudaMalloc(pivot flag)");
-    }
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if ((e = cudaMemsetAsync(h->d_singular, 0, sizeof(unsigned long long), s)) != cudaSuccess)
-        return cuda_fail(e, "cudaMemsetAsync");
-    int rc = frsdg_jac_blocks(h, t, sigma, U, h->d_blocks, stream);
-    if (rc) return rc;
-    if ((e = launch_block_inverse(h->d_blocks, int64_t(nd) * nd, h->d_inv, nd, local_nelem(h), h->d_singular, s)) !=
-        cudaSuccess)
-        return cuda_fail(e, "block-inverse launch");
-    unsigned long long nsing = 0;
-    if ((e = cudaMemcpyAsync(&nsing, h->d_singular, sizeof(nsing), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-        return cuda_fail(e, "pivot flag read");
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(e, "pc setup sync");
-    if (nsing) return fail(FRSDG_ERR_ARG, "frsdg_pc_setup: singular element block (zero pivot)");
-    h->pc_kind = 1;
-    return FRSDG_OK;
+    return run_jac(h, t, sigma, U, JacOut{blocks, 1, nullptr, nullptr, nullptr}, stream);
 }
 
 int frsdg_jac_blocks5(frsdg_handle* h, double t, double sigma, const double* U, double* blocks5, void* stream)
@@ -851,22 +838,50 @@ int frsdg_jac_blocks5(frsdg_handle* h, double t, double sigma, const double* U, 
         return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_jac_blocks5: periodic directions need a multiple of 5 elements");
     if ((reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(blocks5)) & 15)
         return fail(FRSDG_ERR_ARG, "device pointers must be 16-byte aligned");
+    return run_jac(h, t, sigma, U, JacOut{blocks5, 5, nullptr, nullptr, nullptr}, stream);
+}
+
+// The preconditioner's storage (FP32 inverses, the neighbours' entries for the
+// Gauss-Seidel form, the pivot flag), allocated by the first set-up, and its launch.
+static int run_pc_setup(frsdg_handle* h, double t, double sigma, const double* U, bool gs, void* stream)
+{
+    const int nd = h->ndofs;
+    cudaError_t e;
+    const size_t nb = size_t(h->nelem) * nd * nd, no = size_t(h->nelem) * size_t(offdiag_floats(nd));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    h->last = s;
-    Fr2dArgs a = h->a2;
-    a.t = t;
-    a.mode = MODE_JAC;
-    a.jac_cmode = 2;
-    a.cond_sys = h->cfg.cond_sys;
-    a.U = U;
-    a.W = nullptr;
-    a.out = blocks5;
-    a.h = h->cfg.csd_eps;
-    a.inv_h = 1.0 / h->cfg.csd_eps;
-    a.sigma = sigma;
-    const cudaError_t e = dispatch2d<cplx>(h->n, h->cfg.gas_law, h->cfg.riemann, h->geo, a, s);
-    if (e != cudaSuccess) return cuda_fail(e, "Jacobian-block launch");
+    if (!h->d_inv)
+    {
+        if ((e = cudaMalloc(&h->d_inv, sizeof(float) * nb)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(inverse blocks)");
+        // the ghost rows of a row window have no block: z = 0 there
+        if ((e = cudaMemsetAsync(h->d_inv, 0, sizeof(float) * nb, s)) != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
+    }
+    if (gs && !h->d_off && (e = cudaMalloc(&h->d_off, sizeof(float) * no)) != cudaSuccess)
+        return cuda_fail(e, "cudaMalloc(blocks)");
+    if (!h->d_singular && (e = cudaMalloc(&h->d_singular, sizeof(unsigned long long))) != cudaSuccess)
+        return cuda_fail(e, "cudaMalloc(pivot flag)");
+    if ((e = cudaMemsetAsync(h->d_singular, 0, sizeof(unsigned long long), s)) != cudaSuccess)
+        return cuda_fail(e, "cudaMemsetAsync");
+    const int rc = run_jac(h, t, sigma, U, JacOut{nullptr, 0, h->d_inv, gs ? h->d_off : nullptr, h->d_singular}, stream);
+    if (rc) return rc;
+    unsigned long long nsing = 0;
+    if ((e = cudaMemcpyAsync(&nsing, h->d_singular, sizeof(nsing), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+        return cuda_fail(e, "pivot flag read");
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(e, "pc setup sync");
+    if (nsing)
+        return fail(FRSDG_ERR_ARG, gs ? "frsdg_pc_setup_gs: singular element block (zero pivot)"
+                                      : "frsdg_pc_setup: singular element block (zero pivot)");
+    h->pc_kind = gs ? 2 : 1;
     return FRSDG_OK;
+}
+
+int frsdg_pc_setup(frsdg_handle* h, double t, double sigma, const double* U, void* stream)
+{
+    if (!h || !U) return fail(FRSDG_ERR_ARG, "null argument");
+    if (h->cfg.dim != 2) return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_setup: 2D configurations only");
+    if (h->ndofs > kMaxBlockDofs)
+        return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_setup: element blocks above 144 DOFs (p > 5)");
+    if (reinterpret_cast<uintptr_t>(U) & 15) return fail(FRSDG_ERR_ARG, "device pointers must be 16-byte aligned");
+    return run_pc_setup(h, t, sigma, U, false, stream);
 }
 
 int frsdg_pc_setup_gs(frsdg_handle* h, double t, double sigma, const double* U, void* stream)
@@ -875,36 +890,11 @@ int frsdg_pc_setup_gs(frsdg_handle* h, double t, double sigma, const double* U, 
     if (h->cfg.dim != 2) return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_setup_gs: 2D configurations only");
     if (h->cfg.bc[FRSDG_LEFT].kind == FRSDG_BC_PERIODIC || h->cfg.bc[FRSDG_TOP].kind == FRSDG_BC_PERIODIC)
         return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_setup_gs: non-periodic meshes only");
-    const int nd = h->ndofs;
-    if (nd > kMaxBlockDofs) return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_setup_gs: element blocks above 144 DOFs (p > 5)");
-    cudaError_t e;
-    const size_t nb = size_t(h->nelem) * nd * nd;
-    if (!h->d_blocks5)
-    {
-        if ((e = cudaMalloc(&h->d_blocks5, sizeof(double) * 5 * nb)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(blocks)");
-        if ((e = cudaMalloc(&h->d_off, sizeof(float) * 4 * nb)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(blocks)");
-    }
-    if (!h->d_inv && (e = cudaMalloc(&h->d_inv, sizeof(float) * nb)) != cudaSuccess)
-        return cuda_fail(e, "cudaMalloc(inverse blocks)");
-    if (!h->d_singular && (e = cudaMalloc(&h->d_singular, sizeof(unsigned long long))) != cudaSuccess)
-        return cuda_fail(e, "cudaMalloc(pivot flag)");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if ((e = cudaMemsetAsync(h->d_singular, 0, sizeof(unsigned long long), s)) != cudaSuccess)
-        return cuda_fail(e, "cudaMemsetAsync");
-    int rc = frsdg_jac_blocks5(h, t, sigma, U, h->d_blocks5, stream);
-    if (rc) return rc;
-    if ((e = launch_block_inverse(h->d_blocks5, 5 * int64_t(nd) * nd, h->d_inv, nd, h->nelem, h->d_singular, s)) !=
-        cudaSuccess)
-        return cuda_fail(e, "block-inverse launch");
-    if ((e = launch_offdiag_to_f32(h->d_blocks5, h->d_off, nd, h->nelem, s)) != cudaSuccess)
-        return cuda_fail(e, "off-diagonal packing launch");
-    unsigned long long nsing = 0;
-    if ((e = cudaMemcpyAsync(&nsing, h->d_singular, sizeof(nsing), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-        return cuda_fail(e, "pivot flag read");
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(e, "pc setup sync");
-    if (nsing) return fail(FRSDG_ERR_ARG, "frsdg_pc_setup_gs: singular element block (zero pivot)");
-    h->pc_kind = 2;
-    return FRSDG_OK;
+    if (h->ndofs > kMaxBlockDofs)
+        return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_setup_gs: element blocks above 144 DOFs (p > 5)");
+    if (h->win_rows) return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_setup_gs: whole-mesh handles only (no row window)");
+    if (reinterpret_cast<uintptr_t>(U) & 15) return fail(FRSDG_ERR_ARG, "device pointers must be 16-byte aligned");
+    return run_pc_setup(h, t, sigma, U, true, stream);
 }
 
 int frsdg_pc_apply(frsdg_handle* h, const double* r, double* z, void* stream)
@@ -914,8 +904,8 @@ int frsdg_pc_apply(frsdg_handle* h, const double* r, double* z, void* stream)
     if (r == z) return fail(FRSDG_ERR_ARG, "frsdg_pc_apply: z must not alias r");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     h->last = s;
-    const cudaError_t e = h->pc_kind == 2 ? launch_block_gs(h->d_inv, h->d_off, r, z, h->ndofs, h->Nx, h->Ny, s)
-                                          : launch_block_apply(h->d_inv, r, z, h->ndofs, local_nelem(h), s);
+    const cudaError_t e = launch_pc_apply(h->d_inv, h->pc_kind == 2 ? h->d_off : nullptr, r, z, h->n, h->Nx,
+                                          h->win_rows ? h->win_rows : h->Ny, s);
     if (e != cudaSuccess) return cuda_fail(e, "block-apply launch");
     return FRSDG_OK;
 }

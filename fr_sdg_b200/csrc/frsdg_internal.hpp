@@ -18,8 +18,7 @@ enum Mode : int
     MODE_RHS      = 1, // -R(U)                     rhs_func
     MODE_IFUNC    = 2, // U_t + R(M(U))             fun_implicit
     MODE_JVP      = 3, // sigma Im(u)/h + Im(R)/h   ComplexStepJacobianStrategy::matmult
-    MODE_STAGE    = 4, // out = alpha A + beta B + gamma rhs, acc += delta rhs (rhs = -R): one RK stage
-    MODE_JAC      = 5  // element-diagonal blocks of sigma dM/dU + dR(M(U))/dU, coloured complex step
+    MODE_STAGE    = 4  // out = alpha A + beta B + gamma rhs, acc += delta rhs (rhs = -R): one RK stage
 };
 
 // Explicit Runge-Kutta stage fused into the residual's output pass.
@@ -120,8 +119,6 @@ struct Fr2dArgs
     // global row row_base; rows [row_begin, row_end) are computed, the others are ghosts
     int    row_base, row_begin, row_end;
     int    exact_bc;   // complex scalars: differentiate the user-lambda boundary kinds too
-    int    jac_cmode;  // MODE_JAC colouring: 0 checkerboard, 1 three-colour cycles (odd periodic),
-                       // 2 distance-2 colouring (i + 2 j) mod 5 for all five blocks of an element row
     int    in_f64;     // FP32 instantiation: U is an FP64 state, node primitives recovered in FP64
     int    tc;         // FP32 instantiation at n = 5, 6: derivative contractions on the tensor cores
     Ops    ops;
@@ -180,18 +177,6 @@ struct Fr2dBatchArgs
     int stage;                 // SSP-RK3 stage 0, 1, 2
     int mixed;
 };
-
-// Colour of element (gi, gj) for the coloured Jacobian: no two elements sharing a
-// face have the same colour.  Checkerboard, or, when a periodic direction has an
-// odd number of elements, (i mod 2 | 2 for the last) + 3 (j mod 2 | 2 for the last).
-__host__ __device__ inline int elem_colour(int cmode, int Nx, int Ny, int per_x, int per_y, int gi, int gj)
-{
-    if (cmode == 0) return (gi + gj) & 1;
-    if (cmode == 2) return (gi + 2 * gj) % 5;
-    const int cx = (per_x && (Nx & 1) && gi == Nx - 1) ? 2 : (gi & 1);
-    const int cy = (per_y && (Ny & 1) && gj == Ny - 1) ? 2 : (gj & 1);
-    return cx + 3 * cy;
-}
 
 struct Fr1dArgs
 {

@@ -33,11 +33,11 @@ struct frsdg_handle
     double*      d_work = nullptr;   // post-step source copy (WENO)
     double*      d_stage = nullptr;  // host-buffer staging (2 * ntot), allocated on first use
     unsigned long long* d_bad = nullptr;
-    double*      d_blocks = nullptr;  // preconditioner: element-diagonal Jacobian blocks (FP64)
-    float*       d_inv = nullptr;     // and their inverses (FP32); both allocated by the first frsdg_pc_setup
+    // preconditioner, allocated by the first set-up: the FP32 inverses of the element-diagonal
+    // Jacobian blocks, the neighbours' nonzeros (Gauss-Seidel; jac2d.cuh), the pivot flag
+    float*       d_inv = nullptr;
+    float*       d_off = nullptr;
     unsigned long long* d_singular = nullptr;
-    double*      d_blocks5 = nullptr; // block Gauss-Seidel: the five blocks of every element row (FP64)
-    float*       d_off = nullptr;     // and the four off-diagonal ones in FP32; allocated by frsdg_pc_setup_gs
     int          pc_kind = 0;         // 0 none, 1 block Jacobi, 2 block Gauss-Seidel
     double       jvp_t = 0.0, jvp_sigma = 1.0;
     const double* jvp_U = nullptr;

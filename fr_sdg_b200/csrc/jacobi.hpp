@@ -1,4 +1,5 @@
-// jacobi.hpp -- launchers of the element block-Jacobi preconditioner (jacobi.cu).
+// jacobi.hpp -- launchers of the element-block preconditioners: their blocks (jac2d.cuh) and
+// their application (jacobi.cu).
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -10,19 +11,25 @@ namespace frsdg
 // the FP64 block sits in one CTA's shared memory.
 constexpr int kMaxBlockDofs = 144;
 
-size_t block_inverse_smem(int n);
-// inv[e] = inverse of the column-major n x n block blocks[e], in FP32; blocks with
-// a zero pivot are counted in *singular and their inverse is left unwritten.
-// (blocks spaced `stride` doubles apart: n * n for a block-diagonal array, 5 n * n for
-// the diagonal slot of the five blocks of each element row)
-cudaError_t launch_block_inverse(const double* blocks, int64_t stride, float* inv, int n, int64_t n_blocks,
-                                 unsigned long long* singular, cudaStream_t s);
-// off[e][s][.] = (float) blocks5[e][1 + s][.], s = 0..3
-cudaError_t launch_offdiag_to_f32(const double* blocks5, float* off, int n, int64_t nel, cudaStream_t s);
-// One symmetric red-black block Gauss-Seidel sweep z = M^-1 r on an Nx x Ny element grid
-// (no periodic wrap): three launches, red / black / red.
-cudaError_t launch_block_gs(const float* inv, const float* off, const double* r, double* z, int n, int Nx, int Ny,
+// What one launch over the elements' Jacobian blocks leaves (jac2d.cuh): the blocks
+// themselves (blocks, `slots` = 1 or 5 per element), or the FP32 inverses of the diagonal
+// ones and (off not null) the FP32 nonzeros of the neighbours'; blocks with a zero pivot
+// are counted in *singular and their inverse is left unwritten.
+struct JacOut
+{
+    double* blocks;
+    int     slots;
+    float*  inv;
+    float*  off;
+    unsigned long long* singular;
+};
+struct Fr2dArgs;
+template <int N> cudaError_t launch_jac2d(int gas, int riem, const Fr2dArgs& a, const JacOut& o, cudaStream_t s);
+// FP32 values of `off` per element: four neighbours, ND rows, four columns each
+inline int64_t offdiag_floats(int nd) { return int64_t(16) * nd; }
+// z = M^-1 r on an Nx x Ny element grid with n points per direction: the element blocks'
+// inverses alone (off null), or one symmetric red-black block Gauss-Seidel sweep (no
+// periodic wrap; jacobi.cu).
+cudaError_t launch_pc_apply(const float* inv, const float* off, const double* r, double* z, int n, int Nx, int Ny,
                             cudaStream_t s);
-// z[e] = inv[e] r[e] for every element block.
-cudaError_t launch_block_apply(const float* inv, const double* r, double* z, int n, int64_t n_blocks, cudaStream_t s);
 } // namespace frsdg

@@ -193,23 +193,8 @@ template <> struct NodeLoader<cplx>
     {
         const double2 x0 = __ldg(reinterpret_cast<const double2*>(a.U + off));
         const double2 x1 = __ldg(reinterpret_cast<const double2*>(a.U + off + 2));
-        double2 v0, v1;
-        if (a.mode == MODE_JAC)
-        {
-            // seed of this launch slice: DOF d of every element of colour c
-            const int64_t eg = off / a.nd;
-            const int d0 = int(off - eg * a.nd);
-            const int gi = int(eg % a.Nx), gj = int(eg / a.Nx);
-            const int c = int(blockIdx.z) / a.nd, d = int(blockIdx.z) - c * a.nd;
-            const bool on = elem_colour(a.jac_cmode, a.Nx, a.Ny, a.per_x, a.per_y, gi, gj) == c;
-            v0 = make_double2(on && d == d0 ? 1.0 : 0.0, on && d == d0 + 1 ? 1.0 : 0.0);
-            v1 = make_double2(on && d == d0 + 2 ? 1.0 : 0.0, on && d == d0 + 3 ? 1.0 : 0.0);
-        }
-        else
-        {
-            v0 = __ldg(reinterpret_cast<const double2*>(a.W + off));
-            v1 = __ldg(reinterpret_cast<const double2*>(a.W + off + 2));
-        }
+        const double2 v0 = __ldg(reinterpret_cast<const double2*>(a.W + off));
+        const double2 v1 = __ldg(reinterpret_cast<const double2*>(a.W + off + 2));
         s[0] = cplx(x0.x, v0.x * a.h);
         s[1] = cplx(x0.y, v0.y * a.h);
         s[2] = cplx(x1.x, v1.x * a.h);
@@ -557,8 +542,7 @@ __device__ __forceinline__ void stage_epilogue(const Fr2dArgs& a, const Ops& ops
     }
 }
 
-// One tile of the residual pass: tile (bx, by) of element columns/rows (the Jacobian
-// slice of MODE_JAC is blockIdx.z), with the launch arguments `a` and the operators
+// One tile of the residual pass: tile (bx, by) of element columns/rows, with the launch arguments `a` and the operators
 // `ops`; smem_raw is the CTA's dynamic shared memory (T::bytes).
 // FP32 derivatives: the rows of the rounded differentiation matrix do not sum to zero
 // exactly, so a line's constant part (a uniform background flux) would leave a residual
@@ -1060,15 +1044,6 @@ __device__ __forceinline__ void fr2d_tile(const Fr2dArgs& a, const Ops& ops, int
         const S* dyb = sDel + ((e * 4 + 2) * 4 + eq) * N;
         const S* dyt = sDel + ((e * 4 + 3) * 4 + eq) * N;
         const int64_t gbase = (int64_t(j0 + ty) * Nx + (i0 + tx)) * ND + eq;
-        // coloured Jacobian: this slice's column d of the blocks of colour-c elements
-        const int jz = int(blockIdx.z), jc = jz / ND, jd = jz % ND;
-        const int jcol = a.mode == MODE_JAC ? elem_colour(a.jac_cmode, Nx, Ny, a.per_x, a.per_y, i0 + tx, j0 + ty) : 0;
-        const bool jac_store = a.mode == MODE_JAC && (a.jac_cmode == 2 || jcol == jc);
-        // distance-2 colouring: the one element of colour jc in this element's face
-        // neighbourhood sits in slot (jc - colour) mod 5: 0 self, 1 right, 2 top, 3 bottom, 4 left
-        const int64_t jblk = a.jac_cmode == 2
-                                 ? (int64_t(j0 + ty) * Nx + (i0 + tx)) * 5 + (jc - jcol + 5) % 5
-                                 : (int64_t(j0 + ty) * Nx + (i0 + tx));
         S gr[N];
         if constexpr (GEO == GEO_CURVED && !TC)
         {
@@ -1118,9 +1093,7 @@ __device__ __forceinline__ void fr2d_tile(const Fr2dArgs& a, const Ops& ops, int
             {
                 double jv = a.sigma * sSeed[(e * 4 + eq) * NN + l * N + k] * a.inv_h;
                 jv += s_im(R) * a.inv_h;
-                if (a.mode != MODE_JAC) out[gidx] = jv;
-                else if (jac_store)
-                    out[jblk * int64_t(ND * ND) + int64_t(jd) * ND + (l * N + k) * 4 + eq] = jv;
+                out[gidx] = jv;
             }
             else if (a.out_f32)
                 reinterpret_cast<float*>(a.out)[gidx] = static_cast<float>(s_re(R));
@@ -1183,8 +1156,7 @@ cudaError_t launch_fr2d_kernel_v(const Fr2dArgs& a, cudaStream_t st)
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attr_done[dev] = true;
     }
-    dim3 grid((a.Nx + T::TX - 1) / T::TX, (a.row_end - a.row_begin + T::TY - 1) / T::TY,
-              a.mode == MODE_JAC ? (a.jac_cmode == 2 ? 5 : a.jac_cmode ? 9 : 2) * T::NN * 4 : 1);
+    dim3 grid((a.Nx + T::TX - 1) / T::TX, (a.row_end - a.row_begin + T::TY - 1) / T::TY);
     kern<<<grid, T::BT, bytes, st>>>(a);
     return cudaGetLastError();
 }
@@ -1195,7 +1167,7 @@ cudaError_t launch_fr2d_kernel(const Fr2dArgs& a, cudaStream_t st)
     if constexpr (sizeof(S) == 4 && N >= 5 && N <= 8)
     {
         // the FP32 tiles with their derivative contractions on the tensor cores
-        if (a.tc && a.mode != MODE_JAC)
+        if (a.tc)
         {
             if (a.mode == MODE_STAGE && a.post) return launch_fr2d_kernel_v<S, N, GAS, RIEM, GEO, true, true>(a, st);
             return launch_fr2d_kernel_v<S, N, GAS, RIEM, GEO, false, true>(a, st);
