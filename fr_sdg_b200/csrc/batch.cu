@@ -5,8 +5,8 @@
 // correction form a group.  One SSP-RK3 step of the whole batch is a fixed sequence
 // of launches:
 //   for each stage k: one residual+stage launch per group over the concatenated tiles
-//     of its instances (persistent CTAs walking a tile list, batch_stage_args),
-//     then the positivity limiter of that stage's output (one launch per group);
+//     of its instances (persistent CTAs walking a tile list, batch_stage_args), with the
+//     positivity limiter of its output in the epilogue (FP64) or as a launch of its own;
 //   the post-step stabilisation of the last stage into the state (one launch per
 //     group), the limiter of the state, and the clock kernel.
 // Every instance keeps its own time step and final time on the device (BatchClock), so
@@ -57,11 +57,11 @@ cudaError_t stage_launch(int n, int gas, int riem, int var, const Fr2dBatchArgs&
 }
 
 // Tile of the batched residual (elements along x, y) for one order, scalar and variant:
-// the tile_x / tile_y shapes of the single-instance kernel, variant 1 with half the rows.
+// the single-instance kernels' shapes, variant 1 with half the rows.
 void residual_tile(int n, bool f32, int var, int* tx, int* ty)
 {
-    *tx = tile_x(n, 1, f32);
-    const int t = tile_y(n, 1, f32);
+    *tx = f32 ? tile_x(n, 1, true) : line_tile_x(n, false);
+    const int t = f32 ? tile_y(n, 1, true) : line_tile_y(n, false);
     *ty = var == 0 || t == 1 ? t : t / 2;
 }
 
@@ -173,6 +173,7 @@ Fr2dBatchArgs stage_args(const frsdg_batch* b, const Group& g, int var, int k)
     a.ntiles = g.ntiles[var];
     a.stage = k;
     a.mixed = b->mixed;
+    a.limit = !b->mixed && g.any_pp;
     return a;
 }
 
@@ -209,7 +210,7 @@ cudaError_t enqueue_step(const frsdg_batch* b, cudaStream_t s)
         for (const Group& g : b->groups)
             if ((e = launch_stage(b, g, g.var, g.grid, k, s)) != cudaSuccess) return e;
         for (const Group& g : b->groups)
-            if ((k < 2 ? g.any_pp : g.unfused) && (e = launch_pp(b, g, k, s)) != cudaSuccess) return e;
+            if (b->mixed && (k < 2 ? g.any_pp : g.unfused) && (e = launch_pp(b, g, k, s)) != cudaSuccess) return e;
     }
     for (const Group& g : b->groups)
     {
@@ -440,13 +441,14 @@ int frsdg_batch_create(frsdg_handle* const* handles, int32_t count, double* cons
             // runs an element-local post-step (filter) and yields the wave speed
             const bool pp_on = h->cfg.pp_limit != 0;
             const bool fused = h->cfg.apply_filter || !h->cfg.apply_weno;
-            // (the first two stages' limiter runs as its own pass: measured faster than
-            // the epilogue on the 1024^2 p = 5 blast, 2.44 against 2.70 ms per stage)
-            in.post[0] = in.post[1] = 0;
+            // (FP64: every stage's limiter is its epilogue, as in frsdg_rk_stage_fused; the
+            // FP32 tiles' first two stages are limited by a pass of their own)
+            const int lim = pp_on && !b->mixed ? POST_PP : 0;
+            in.post[0] = in.post[1] = lim;
             in.fused_step = fused ? 1 : 0;
             in.post[2] = fused ? (pp_on ? POST_PP : 0) | (h->cfg.apply_filter ? POST_FILTER : 0) |
                                      (dt_scale ? POST_AMAX : 0)
-                               : 0;
+                               : lim;
             if (pp_on) g.any_pp = 1;
             const size_t nt = size_t(h->ntot);
             for (int k = 0; k < 3; ++k)

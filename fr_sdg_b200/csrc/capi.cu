@@ -732,9 +732,10 @@ int frsdg_rk_stage_fused(frsdg_handle* h, double t, const double* Us, const doub
     // the post-step is element-local unless it is the WENO limiter alone (the filter
     // overrides WENO when both are set)
     const bool local_step = h->cfg.apply_filter || !h->cfg.apply_weno;
-    // the limiter alone after a stage runs as its own pass (measured faster than the
-    // epilogue on the 1024^2 p = 5 blast: 2.44 against 2.70 ms per stage)
-    if (h->cfg.dim == 2 && step && local_step)
+    // the limiter alone after a stage: in the epilogue of the FP64 line tiles, whose threads
+    // hold the stage's values (512^2 p = 5 blast: 0.29 ms against 0.25 + 0.075); its own pass after the FP32
+    // tiles (1024^2: 2.44 against 2.70 ms per stage in their epilogue)
+    if (h->cfg.dim == 2 && (step ? local_step : limit && !mixed))
     {
         int post = limit ? POST_PP : 0;
         if (step && h->cfg.apply_filter) post |= POST_FILTER;

@@ -73,18 +73,21 @@ __device__ __forceinline__ bool positive_in_float_range(double x)
 static __device__ __noinline__ double ieee_sqrt(double x) { return sqrt(x); }
 static __device__ __noinline__ double ieee_rcp(double x) { return 1.0 / x; }
 
-// sqrt in FP64: single-precision reciprocal square root seed, two Newton steps
-// y <- y (3 - x y^2) / 2 for 1/sqrt(x), then s = x y with one Heron correction
-// s <- s + (x - s^2) y / 2 (Karp and Markstein, ACM TOMS 23(4), 1997).  Inputs
-// outside [2^-122, 2^123) (zero, negatives, subnormals, inf, NaN) take the IEEE
-// square root.
+// sqrt in FP64 from the hardware's approximate FP64 reciprocal square root y
+// (rsqrt.approx.f64 of the PTX ISA, the leading 32 bits): with g = x y ~ sqrt(x) and
+// h = y / 2, one coupled Newton step r = 1/2 - g h, g <- g + g r, h <- h + h r, then a Heron
+// correction g + (x - g^2) h (Markstein, IBM J. Res. Dev. 34(1), 1990): the seed's error is
+// squared twice.  Inputs outside [2^-122, 2^123) (zero, negatives, subnormals, inf, NaN)
+// take the IEEE square root.
 __device__ __forceinline__ double sqrt_fast(double x)
 {
-    double y = static_cast<double>(rsqrtf(static_cast<float>(x)));
-    y = y * fma(-0.5 * x, y * y, 1.5);
-    y = y * fma(-0.5 * x, y * y, 1.5);
-    const double s = x * y;
-    return fma(fma(-s, s, x), 0.5 * y, s);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y;
+    const double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    return fma(fma(-g, g, x), h, g);
 }
 __device__ __forceinline__ double s_sqrt(double x)
 {
@@ -112,20 +115,16 @@ __device__ __forceinline__ cplx s_exp(cplx z)
     return {m * c, m * s};
 }
 
-// reciprocal: 1/x.  In FP64 the hardware's approximate single-precision reciprocal
-// (rcp.approx, at most one FP32 ulp off by the PTX ISA) seeds two Newton-Raphson
-// steps r <- r + r (1 - x r) (error below 2^-90 before rounding, so within 2 ulp of the
-// correctly rounded value; Markstein, IBM J. Res. Dev. 34(1), 1990).  Inputs outside
-// [2^-122, 2^123) in magnitude take the IEEE division.  (Against a correctly rounded FP32
-// seed: the same results on the 1024^2 p = 5 residual, 2.4 % less time.)
+// reciprocal: 1/x.  In FP64 the hardware's approximate FP64 reciprocal r (rcp.approx.f64 of
+// the PTX ISA, the leading 32 bits) and one third-order step r + r (e + e^2), e = 1 - x r
+// (the seed's error cubed; Markstein, IBM J. Res. Dev. 34(1), 1990).  Inputs outside
+// [2^-122, 2^123) in magnitude take the IEEE division.
 __device__ __forceinline__ double rcp_fast(double x)
 {
-    float sf;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(sf) : "f"(static_cast<float>(x)));
-    double r = static_cast<double>(sf);
-    r = fma(r, fma(-x, r, 1.0), r);
-    r = fma(r, fma(-x, r, 1.0), r);
-    return r;
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
 }
 __device__ __forceinline__ double s_rcp(double x)
 {
@@ -134,6 +133,24 @@ __device__ __forceinline__ double s_rcp(double x)
 }
 __device__ __forceinline__ float s_rcp(float x) { return 1.0f / x; }
 __device__ __forceinline__ cplx s_rcp(cplx z) { return cplx(1.0) / z; }
+
+// wrap_positive (macro_and_libc.hpp:117-138): max(DBL_MIN, rho); for complex, the
+// real part decides and a clamped value loses its imaginary part.
+__device__ __forceinline__ double s_wrap_positive(double r)
+{
+    const double floor = 2.2250738585072014e-308; // DBL_MIN
+    return fmax(floor, r);
+}
+__device__ __forceinline__ float s_wrap_positive(float r)
+{
+    const float floor = 1.17549435e-38f; // FLT_MIN
+    return fmaxf(floor, r);
+}
+__device__ __forceinline__ cplx s_wrap_positive(cplx r)
+{
+    const double floor = 2.2250738585072014e-308;
+    return (r.re < floor) ? cplx(floor, 0.0) : r;
+}
 
 // Math policies of the physics helpers.  MathChecked: s_rcp and s_sqrt.  MathDeferred:
 // in FP64 the fast paths alone, each recording in `bad` whether its input lay outside
@@ -146,18 +163,27 @@ struct MathChecked
 {
     template <class S> __device__ __forceinline__ S rcp(S x) const { return s_rcp(x); }
     template <class S> __device__ __forceinline__ S sqrt(S x) const { return s_sqrt(x); }
+    template <class S> __device__ __forceinline__ S wrap(S x) const { return s_wrap_positive(x); }
 };
 struct MathDeferred
 {
     unsigned& bad;
+    // wrap_positive leaves normal positive finite values as they are; others are recorded
+    __device__ __forceinline__ double wrap(double x) const
+    {
+        if (static_cast<unsigned>(__double2hiint(x)) - 0x00100000u >= 0x7fe00000u) bad = 1u;
+        return x;
+    }
+    __device__ __forceinline__ float wrap(float x) const { return s_wrap_positive(x); }
+    __device__ __forceinline__ cplx wrap(cplx x) const { return s_wrap_positive(x); }
     __device__ __forceinline__ double rcp(double x) const
     {
-        bad |= in_float_range(x) ? 0u : 1u;
+        if (!in_float_range(x)) bad = 1u;
         return rcp_fast(x);
     }
     __device__ __forceinline__ double sqrt(double x) const
     {
-        bad |= positive_in_float_range(x) ? 0u : 1u;
+        if (!positive_in_float_range(x)) bad = 1u;
         return sqrt_fast(x);
     }
     // FP32: the hardware approximations with one Newton step (within 2 ulp of the IEEE
@@ -192,24 +218,6 @@ __device__ __forceinline__ double s_im(cplx z) { return z.im; }
 __device__ __forceinline__ double s_branch(double x) { return x; }
 __device__ __forceinline__ double s_branch(float x) { return x; }
 __device__ __forceinline__ double s_branch(cplx z) { return z.re + z.im; }
-
-// wrap_positive (macro_and_libc.hpp:117-138): max(DBL_MIN, rho); for complex, the
-// real part decides and a clamped value loses its imaginary part.
-__device__ __forceinline__ double s_wrap_positive(double r)
-{
-    const double floor = 2.2250738585072014e-308; // DBL_MIN
-    return fmax(floor, r);
-}
-__device__ __forceinline__ float s_wrap_positive(float r)
-{
-    const float floor = 1.17549435e-38f; // FLT_MIN
-    return fmaxf(floor, r);
-}
-__device__ __forceinline__ cplx s_wrap_positive(cplx r)
-{
-    const double floor = 2.2250738585072014e-308;
-    return (r.re < floor) ? cplx(floor, 0.0) : r;
-}
 
 template <class S> __device__ __forceinline__ S s_select(bool c, S a, S b) { return c ? a : b; }
 

@@ -176,6 +176,7 @@ struct Fr2dBatchArgs
     int ntiles;
     int stage;                 // SSP-RK3 stage 0, 1, 2
     int mixed;
+    int limit;                 // FP64: an instance limits every stage output (BatchInst2D::post)
 };
 
 struct Fr1dArgs
@@ -223,6 +224,23 @@ __host__ __device__ constexpr int tile_y(int n, int words, bool f32)
     if (face_tiles(n, words, f32)) return n == 5 ? 2 : n == 6 ? 4 : n <= 9 ? 2 : 1;
     return n <= 2 ? 8 : n <= 3 ? 4 : n <= 4 ? 4 : n <= 6 ? 2 : n <= 9 ? 2 : 1;
 #endif
+}
+
+// Tile of the FP64 residual with one thread per line of nodes (line2d.cuh): TX TY n
+// threads, whole warps or nearly, with a halo of at most half the tile.  Measured on the
+// 1024^2 blast (p = 8, 9: 640^2), times against the node-per-thread tiles this kernel
+// replaced: p = 1 0.16 -> 0.05 (640^2), p = 2 0.48 -> 0.26, p = 3 0.80 -> 0.34, p = 4 1.08 ->
+// 0.53 (8 x 4: five full warps; 4 x 4 0.60), p = 5 1.23 -> 0.73 (8 x 4 0.79, 4 x 8 0.82, 2 x 8
+// 0.81, 5 x 2 0.83), p = 6 2.25 -> 1.08, p = 7 0.70 -> 0.35 (512^2), p = 8 1.22 -> 0.90, p = 9
+// 1.67 -> 1.21 ms.  Curved meshes keep both fluxes in shared memory: 3 x 2 at n >= 9 (p = 8
+// 240^2 vortex 0.31 -> 0.23 ms; 4 x 4 0.33).
+__host__ __device__ constexpr int line_tile_x(int n, bool curved)
+{
+    return n <= 3 || n == 5 ? 8 : curved && n >= 9 ? 3 : 4;
+}
+__host__ __device__ constexpr int line_tile_y(int n, bool curved)
+{
+    return n <= 2 ? 8 : curved && n >= 9 ? 2 : 4;
 }
 
 // Launchers (one translation unit per polynomial order).

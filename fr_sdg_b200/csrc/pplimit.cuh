@@ -94,17 +94,52 @@ template <class PA> __device__ __forceinline__ double node_wave_speed_fast(const
     return s_sqrt(v2) + s_sqrt(fmax(c2, 0.0));
 }
 
+// pp_pressure with reciprocals
+template <int NV, class PA> __device__ __forceinline__ double pp_pressure_rcp(const PA& a, const double* u)
+{
+    double m2 = 0.0;
+#pragma unroll
+    for (int c = 1; c < NV - 1; ++c) m2 += u[c] * u[c];
+    const double rho_e = u[NV - 1] - 0.5 * m2 * s_rcp(u[0]);
+    if (a.gas_law == FRSDG_GAS_IDEAL) return (a.gas.gamma - 1.0) * rho_e;
+    const double arr = a.gas.a * u[0] * u[0];
+    return ((a.gas.gamma - 1.0) * (rho_e + arr)) * s_rcp(1.0 - a.gas.b * u[0]) - arr;
+}
+
+// The admissible end of the segment ub -> uq at pressure eps: p - eps is positive at ub and
+// negative (or not a number) at uq; the bracket [lo, hi] is narrowed to rounding by the
+// Illinois form of the secant rule (Dowell and Jarratt, BIT 11, 1971), with a bisection every
+// third step and wherever the secant fails, and its admissible end returned.  A dozen
+// pressures instead of the sixty of plain bisection: the limiter's elements set the run time
+// of a pass over a shocked state (a batched 32^2 to 96^2 explosion step, 24 instances).
 template <int NV, class PA>
 __device__ __forceinline__ double pp_segment_root(const PA& a, const double* ub, const double* uq, double eps)
 {
     double lo = 0.0, hi = 1.0, s[NV];
-    for (int it = 0; it < 60; ++it)
+    double flo = pp_pressure_rcp<NV>(a, ub) - eps, fhi = uq[0] > 0.0 ? pp_pressure_rcp<NV>(a, uq) - eps : -1e300;
+    int last = 0;
+    for (int it = 0; it < 60 && hi - lo > 2.0e-16 * hi; ++it)
     {
-        const double mid = 0.5 * (lo + hi);
+        double mid = lo + (hi - lo) * (flo / (flo - fhi));
+        if (it % 3 == 2 || !(mid > lo && mid < hi)) mid = 0.5 * (lo + hi);
+        if (!(mid > lo && mid < hi)) break;  // neighbours in floating point
 #pragma unroll
         for (int c = 0; c < NV; ++c) s[c] = ub[c] + mid * (uq[c] - ub[c]);
-        if (s[0] > 0.0 && pp_pressure<NV>(a, s) >= eps) lo = mid;
-        else hi = mid;
+        const double f = s[0] > 0.0 ? pp_pressure_rcp<NV>(a, s) - eps : -1e300;
+        if (f >= 0.0)
+        {
+            lo = mid;
+            flo = f;
+            if (last == 1) fhi *= 0.5;
+            last = 1;
+        }
+        else
+        {
+            hi = mid;
+            fhi = f;
+            if (last == -1) flo *= 0.5;
+            last = -1;
+        }
     }
     return lo;
 }

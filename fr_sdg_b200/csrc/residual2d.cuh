@@ -390,6 +390,11 @@ __device__ __forceinline__ void face_ghost(const Fr2dArgs& a, int i0, int j0, Fa
     }
 }
 
+} // namespace frsdg
+#include "line2d.cuh"
+namespace frsdg
+{
+
 // Jumps scale*(F* - F.n) of the tile sides of a face point; F.n from the cached
 // volume fluxes (F.n = F on affine x-faces, G on affine y-faces).
 template <class S, int N, int GEO, bool XF, class T>
@@ -1143,26 +1148,16 @@ cudaError_t launch_fr2d_kernel_v(const Fr2dArgs& a, cudaStream_t st)
     using T = Tile2D<S, N, GEO, 0, TC>;
     auto kern = fr2d_kernel<S, N, GAS, RIEM, GEO, POST, TC>;
     constexpr size_t bytes = POST ? T::bytes_post : T::bytes_launch;
-    // kernel attributes are per device: set them once on each device that launches
-    static bool attr_done[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    static bool done[64] = {};
+    const cudaError_t e = set_smem_once(kern, bytes, done);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !attr_done[dev])
-    {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) attr_done[dev] = true;
-    }
     dim3 grid((a.Nx + T::TX - 1) / T::TX, (a.row_end - a.row_begin + T::TY - 1) / T::TY);
     kern<<<grid, T::BT, bytes, st>>>(a);
     return cudaGetLastError();
 }
 
 template <class S, int N, int GAS, int RIEM, int GEO>
-cudaError_t launch_fr2d_kernel(const Fr2dArgs& a, cudaStream_t st)
+cudaError_t launch_fr2d_tiles(const Fr2dArgs& a, cudaStream_t st)
 {
     if constexpr (sizeof(S) == 4 && N >= 5 && N <= 8)
     {
@@ -1178,6 +1173,14 @@ cudaError_t launch_fr2d_kernel(const Fr2dArgs& a, cudaStream_t st)
         if (a.mode == MODE_STAGE && a.post) return launch_fr2d_kernel_v<S, N, GAS, RIEM, GEO, true>(a, st);
     }
     return launch_fr2d_kernel_v<S, N, GAS, RIEM, GEO, false>(a, st);
+}
+
+// FP64: one thread per line of nodes (line2d.cuh); complex and FP32: these tiles.
+template <class S, int N, int GAS, int RIEM, int GEO>
+cudaError_t launch_fr2d_kernel(const Fr2dArgs& a, cudaStream_t st)
+{
+    if constexpr (std::is_same<S, double>::value) return launch_line<N, GAS, RIEM, GEO>(a, st);
+    else return launch_fr2d_tiles<S, N, GAS, RIEM, GEO>(a, st);
 }
 
 // ---- batches ------------------------------------------------------------------
@@ -1264,35 +1267,64 @@ fr2d_batch_kernel(const __grid_constant__ Fr2dBatchArgs b)
     }
 }
 
+// The same walk with the FP64 line tiles.
+template <int N, int GAS, int RIEM, int VAR, bool POST>
+__global__ void __launch_bounds__((Line2D<N, GEO_AFFINE, VAR>::BT), (Line2D<N, GEO_AFFINE, VAR>::CTAS))
+    fr2d_line_batch_kernel(const __grid_constant__ Fr2dBatchArgs b)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ __align__(16) unsigned long long sa_raw[(sizeof(Fr2dArgs) + 7) / 8];
+    Fr2dArgs& sa = *reinterpret_cast<Fr2dArgs*>(sa_raw);
+    constexpr int HEAD = int(offsetof(Fr2dArgs, ops) / 8);  // the arguments before the operators
+    for (int tile = blockIdx.x; tile < b.ntiles; tile += gridDim.x)
+    {
+        const int4 tm = b.tiles[tile];
+        const BatchInst2D& in = b.inst[tm.x];
+        const BatchClock ck = b.clock[in.inst];
+        if (!ck.active) continue;  // uniform over the CTA
+        __syncthreads();           // the previous tile is done with sa
+        const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&in.a);
+        for (int q = threadIdx.x; q < HEAD; q += blockDim.x) sa_raw[q] = src[q];
+        __syncthreads();
+        if (threadIdx.x == 0) batch_stage_args(sa, in, ck, b.stage, b.mixed != 0);
+        __syncthreads();
+        fr2d_line_tile<N, GAS, RIEM, GEO_AFFINE, VAR, POST>(sa, b.ops, tm.y, tm.z, smem_raw);
+    }
+}
+
 // POST: the instantiation with the stage epilogue, for the stage that carries a post-step
 // (the last); the others skip the epilogue's registers and spills.
+template <class K>
+cudaError_t launch_batch_kernel(K kern, int threads, size_t bytes, bool (&done)[64], const Fr2dBatchArgs& b, int grid,
+                                cudaStream_t st, int* occupancy)
+{
+    const cudaError_t e = set_smem_once(kern, bytes, done);
+    if (e != cudaSuccess) return e;
+    if (occupancy) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy, kern, threads, bytes);
+    if (grid > 0 && b.ntiles > 0) kern<<<grid, threads, bytes, st>>>(b);
+    return cudaGetLastError();
+}
 template <class S, int N, int GAS, int RIEM, int VAR, bool POST>
 cudaError_t launch_fr2d_batch_kernel_v(const Fr2dBatchArgs& b, int grid, cudaStream_t st, int* occupancy)
 {
-    using T = Tile2D<S, N, GEO_AFFINE, VAR>;
-    auto kern = fr2d_batch_kernel<S, N, GAS, RIEM, VAR, POST>;
-    constexpr size_t bytes = POST ? T::bytes_post : T::bytes_launch;
-    static bool attr_done[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !attr_done[dev])
+    static bool done[64] = {};
+    if constexpr (std::is_same<S, double>::value)
     {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) attr_done[dev] = true;
+        using T = Line2D<N, GEO_AFFINE, VAR>;
+        return launch_batch_kernel(fr2d_line_batch_kernel<N, GAS, RIEM, VAR, POST>, T::BT, T::bytes, done, b, grid, st, occupancy);
     }
-    if (occupancy) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy, kern, T::BT, bytes);
-    if (grid > 0 && b.ntiles > 0) kern<<<grid, T::BT, bytes, st>>>(b);
-    return cudaGetLastError();
+    else
+    {
+        using T = Tile2D<S, N, GEO_AFFINE, VAR>;
+        return launch_batch_kernel(fr2d_batch_kernel<S, N, GAS, RIEM, VAR, POST>, T::BT,
+                                   POST ? T::bytes_post : T::bytes_launch, done, b, grid, st, occupancy);
+    }
 }
 
 template <class S, int N, int GAS, int RIEM, int VAR>
 cudaError_t launch_fr2d_batch_kernel(const Fr2dBatchArgs& b, int grid, cudaStream_t st, int* occupancy)
 {
-    if (b.stage == 2) return launch_fr2d_batch_kernel_v<S, N, GAS, RIEM, VAR, true>(b, grid, st, occupancy);
+    if (b.stage == 2 || b.limit) return launch_fr2d_batch_kernel_v<S, N, GAS, RIEM, VAR, true>(b, grid, st, occupancy);
     return launch_fr2d_batch_kernel_v<S, N, GAS, RIEM, VAR, false>(b, grid, st, occupancy);
 }
 
