@@ -37,8 +37,11 @@ def _nvcc() -> str:
 
 def _units() -> list[tuple[Path, Path, list[str]]]:
     units = []
-    for n in N_VALUES:
-        units.append((CSRC / "instances.cu", BUILD / f"instances_n{n}.o", [f"-DFRSDG_N={n}"]))
+    # two parts per order, the largest first: the build's wall time is its longest unit
+    for n in reversed(N_VALUES):
+        for part in (0, 1):
+            units.append((CSRC / "instances.cu", BUILD / f"instances_n{n}_{part}.o",
+                          [f"-DFRSDG_N={n}", f"-DFRSDG_PART={part}"]))
     for name in ("capi.cu", "stab.cu", "setup_ops.cpp", "noalloc.cu", "jacobi.cu", "petsc_io.cu", "pplimit.cu", "batch.cu", "tc.cu", "krylov.cu"):
         units.append((CSRC / name, BUILD / (Path(name).stem + ".o"), []))
     return units

@@ -3,6 +3,8 @@
 // The residual is templated on its scalar S:
 //   double  the FP64 residual (rhs_func / fun_implicit),
 //   cplx    complex FP64 for the complex-step JVP (matmult of the reference),
+//   dual    value and directional derivative in FP64: the complex step's limit h -> 0, which
+//           takes the place of cplx when h^2 is below rounding (csd_eps <= 1e-20);
 //   float   the FP32 residual of the mixed-precision form.
 // cplx follows std::complex<double> semantics for finite values: principal-branch
 // sqrt, Smith's division (R. L. Smith, "Algorithm 116: Complex division",
@@ -53,6 +55,26 @@ __device__ __forceinline__ cplx operator/(double s, cplx b) { return cplx(s) / b
 __device__ __forceinline__ cplx& operator+=(cplx& a, cplx b) { a = a + b; return a; }
 __device__ __forceinline__ cplx& operator-=(cplx& a, cplx b) { a = a - b; return a; }
 
+// Value and derivative (re, im as in cplx): the products' second-order terms, h^2 smaller
+// than the first-order ones, are left out, and a quotient needs one reciprocal.
+struct __align__(16) dual
+{
+    double re, im;
+    __host__ __device__ constexpr dual() : re(0.0), im(0.0) {}
+    __host__ __device__ constexpr dual(double r) : re(r), im(0.0) {}
+    __host__ __device__ constexpr dual(double r, double i) : re(r), im(i) {}
+};
+__device__ __forceinline__ dual operator+(dual a, dual b) { return {a.re + b.re, a.im + b.im}; }
+__device__ __forceinline__ dual operator-(dual a, dual b) { return {a.re - b.re, a.im - b.im}; }
+__device__ __forceinline__ dual operator-(dual a) { return {-a.re, -a.im}; }
+__device__ __forceinline__ dual operator*(dual a, dual b) { return {a.re * b.re, fma(a.re, b.im, a.im * b.re)}; }
+__device__ __forceinline__ dual operator*(double s, dual a) { return {s * a.re, s * a.im}; }
+__device__ __forceinline__ dual operator*(dual a, double s) { return {a.re * s, a.im * s}; }
+__device__ __forceinline__ dual operator+(dual a, double s) { return {a.re + s, a.im}; }
+__device__ __forceinline__ dual operator+(double s, dual a) { return {s + a.re, a.im}; }
+__device__ __forceinline__ dual operator-(dual a, double s) { return {a.re - s, a.im}; }
+__device__ __forceinline__ dual operator-(double s, dual a) { return {s - a.re, -a.im}; }
+
 // ---- generic scalar functions -------------------------------------------
 // Exponent tests of the fast paths: |x| (or x, positive) in [2^-122, 2^123), well
 // inside the range of normal floats, by the biased exponent with integer operations
@@ -89,6 +111,19 @@ __device__ __forceinline__ double sqrt_fast(double x)
     h = fma(h, r, h);
     return fma(fma(-g, g, x), h, g);
 }
+// the same with h = 1 / (2 sqrt(x)) to full precision
+__device__ __forceinline__ double sqrt_fast(double x, double& h_out)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y;
+    const double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    g = fma(fma(-g, g, x), h, g);
+    h_out = fma(h, fma(-g, h, 0.5) * 2.0, h);
+    return g;
+}
 __device__ __forceinline__ double s_sqrt(double x)
 {
     if (!positive_in_float_range(x)) return ieee_sqrt(x);
@@ -103,9 +138,29 @@ __device__ __forceinline__ cplx s_sqrt(cplx z)
     if (z.re >= 0.0) return {t, z.im / (2.0 * t)};
     return {fabs(z.im) / (2.0 * t), copysign(t, z.im)};
 }
+// as the complex root to first order: principal branch, 0 at 0
+__device__ __forceinline__ dual s_sqrt(dual z)
+{
+    if (positive_in_float_range(z.re))
+    {
+        double h;
+        const double g = sqrt_fast(z.re, h);
+        return {g, z.im * h};
+    }
+    if (z.re == 0.0 && z.im == 0.0) return {0.0, z.im};
+    const double t = ieee_sqrt(fabs(z.re));
+    if (z.re >= 0.0) return {t, z.im / (2.0 * t)};
+    return {fabs(z.im) / (2.0 * t), copysign(t, z.im)};
+}
 __device__ __forceinline__ double s_log(double x) { return log(x); }
 __device__ __forceinline__ cplx s_log(cplx z) { return {log(hypot(z.re, z.im)), atan2(z.im, z.re)}; }
+__device__ __forceinline__ dual s_log(dual z) { return {log(z.re), z.im / z.re}; }
 __device__ __forceinline__ double s_exp(double x) { return exp(x); }
+__device__ __forceinline__ dual s_exp(dual z)
+{
+    const double m = exp(z.re);
+    return {m, m * z.im};
+}
 __device__ __forceinline__ float s_exp(float x) { return expf(x); }
 __device__ __forceinline__ cplx s_exp(cplx z)
 {
@@ -133,6 +188,18 @@ __device__ __forceinline__ double s_rcp(double x)
 }
 __device__ __forceinline__ float s_rcp(float x) { return 1.0f / x; }
 __device__ __forceinline__ cplx s_rcp(cplx z) { return cplx(1.0) / z; }
+__device__ __forceinline__ dual s_rcp(dual z)
+{
+    const double r = s_rcp(z.re);
+    return {r, -(z.im * r) * r};
+}
+__device__ __forceinline__ dual operator/(dual a, dual b)
+{
+    const double q = a.re / b.re;
+    return {q, (a.im - q * b.im) / b.re};
+}
+__device__ __forceinline__ dual operator/(dual a, double s) { return {a.re / s, a.im / s}; }
+__device__ __forceinline__ dual operator/(double s, dual b) { return dual(s) / b; }
 
 // wrap_positive (macro_and_libc.hpp:117-138): max(DBL_MIN, rho); for complex, the
 // real part decides and a clamped value loses its imaginary part.
@@ -150,6 +217,11 @@ __device__ __forceinline__ cplx s_wrap_positive(cplx r)
 {
     const double floor = 2.2250738585072014e-308;
     return (r.re < floor) ? cplx(floor, 0.0) : r;
+}
+__device__ __forceinline__ dual s_wrap_positive(dual r)
+{
+    const double floor = 2.2250738585072014e-308;
+    return (r.re < floor) ? dual(floor, 0.0) : r;
 }
 
 // Math policies of the physics helpers.  MathChecked: s_rcp and s_sqrt.  MathDeferred:
@@ -176,6 +248,19 @@ struct MathDeferred
     }
     __device__ __forceinline__ float wrap(float x) const { return s_wrap_positive(x); }
     __device__ __forceinline__ cplx wrap(cplx x) const { return s_wrap_positive(x); }
+    __device__ __forceinline__ dual wrap(dual x) const { return {wrap(x.re), x.im}; }
+    __device__ __forceinline__ dual rcp(dual x) const
+    {
+        const double r = rcp(x.re);
+        return {r, -(x.im * r) * r};
+    }
+    __device__ __forceinline__ dual sqrt(dual x) const
+    {
+        if (!positive_in_float_range(x.re)) bad = 1u;
+        double h;
+        const double t = sqrt_fast(x.re, h);
+        return {t, x.im * h};
+    }
     __device__ __forceinline__ double rcp(double x) const
     {
         if (!in_float_range(x)) bad = 1u;
@@ -215,6 +300,9 @@ __device__ __forceinline__ double s_re(double x) { return x; }
 __device__ __forceinline__ double s_re(float x) { return x; }
 __device__ __forceinline__ double s_re(cplx z) { return z.re; }
 __device__ __forceinline__ double s_im(cplx z) { return z.im; }
+__device__ __forceinline__ double s_re(dual z) { return z.re; }
+__device__ __forceinline__ double s_im(dual z) { return z.im; }
+__device__ __forceinline__ double s_branch(dual z) { return z.re; }
 __device__ __forceinline__ double s_branch(double x) { return x; }
 __device__ __forceinline__ double s_branch(float x) { return x; }
 __device__ __forceinline__ double s_branch(cplx z) { return z.re + z.im; }
@@ -238,6 +326,11 @@ template <> struct scalar_traits<float>
 {
     using real = float;
     static constexpr int words = 1;
+};
+template <> struct scalar_traits<dual>
+{
+    using real = double;
+    static constexpr int words = 2;
 };
 template <> struct scalar_traits<cplx>
 {

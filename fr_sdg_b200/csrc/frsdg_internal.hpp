@@ -194,6 +194,9 @@ struct Fr1dArgs
     double h, inv_h, sigma;
     unsigned long long* bad;
     StageArgs st;
+    int    post, pad_post_;  // MODE_STAGE: POST_FILTER, POST_PP on the stage output
+    double w[kMaxN];         // GLL weights and floor of the positivity limiter
+    double pp_eps;
     Ops    ops;
 };
 

@@ -50,27 +50,27 @@ template <int N> struct Jac2D
 
 // The seeded complex state of one node: U + i h e_var (var < 0: no seed), through M for
 // the change of variables (NodeLoader<cplx> of the JVP on the same seed).
-__device__ __forceinline__ void jac_load(const Fr2dArgs& a, int64_t off, int var, cplx s[4])
+template <class C> __device__ __forceinline__ void jac_load(const Fr2dArgs& a, int64_t off, int var, C s[4])
 {
     const double2 x0 = __ldg(reinterpret_cast<const double2*>(a.U + off));
     const double2 x1 = __ldg(reinterpret_cast<const double2*>(a.U + off + 2));
-    s[0] = cplx(x0.x, var == 0 ? a.h : 0.0);
-    s[1] = cplx(x0.y, var == 1 ? a.h : 0.0);
-    s[2] = cplx(x1.x, var == 2 ? a.h : 0.0);
-    s[3] = cplx(x1.y, var == 3 ? a.h : 0.0);
+    s[0] = C(x0.x, var == 0 ? a.h : 0.0);
+    s[1] = C(x0.y, var == 1 ? a.h : 0.0);
+    s[2] = C(x1.x, var == 2 ? a.h : 0.0);
+    s[3] = C(x1.y, var == 3 ? a.h : 0.0);
     if (a.cond_sys)
     {
-        const cplx rho  = s_exp(s[0]);
-        const cplx ssq  = (cplx(0.0) + s[1] * s[1]) + s[2] * s[2];
-        const cplx rhoE = rho * (s_exp(s[3]) + 0.5 * ssq);
-        const cplx u = s[1], v = s[2];
+        const C rho  = s_exp(s[0]);
+        const C ssq  = (C(0.0) + s[1] * s[1]) + s[2] * s[2];
+        const C rhoE = rho * (s_exp(s[3]) + 0.5 * ssq);
+        const C u = s[1], v = s[2];
         s[0] = rho; s[1] = rho * u; s[2] = rho * v; s[3] = rhoE;
     }
 }
 
-template <int GAS> __device__ __forceinline__ void jac_record(const GasParams& g, const cplx s[4], cplx rec[RF_N])
+template <int GAS, class C> __device__ __forceinline__ void jac_record(const GasParams& g, const C s[4], C rec[RF_N])
 {
-    const NodePrim<cplx> pr = node_prim<GAS>(g, s[0], s[1], s[2], s[3]);
+    const NodePrim<C> pr = node_prim<GAS>(g, s[0], s[1], s[2], s[3]);
     rec[RF_RHO] = s[0];
     rec[RF_E] = s[3];
     rec[RF_U] = pr.u;
@@ -80,7 +80,7 @@ template <int GAS> __device__ __forceinline__ void jac_record(const GasParams& g
 }
 
 // The derivatives of element (gi, gj) into shared memory (Jac2D layout).
-template <int N, int GAS, int RIEM>
+template <class C, int N, int GAS, int RIEM>
 __device__ __forceinline__ void jac_derivatives(const Fr2dArgs& a, int gi, int gj, double* sm)
 {
     using J = Jac2D<N>;
@@ -100,11 +100,11 @@ __device__ __forceinline__ void jac_derivatives(const Fr2dArgs& a, int gi, int g
     for (int q = tid; q < NN * 4; q += kJacThreads)
     {
         const int node = q >> 2, var = q & 3;
-        cplx s[4];
+        C s[4];
         jac_load(a, base + node * 4, var, s);
         if (var == 0 && !density_ok(s[0].re) && a.bad) atomicAdd(a.bad, 1ull);
-        const NodePrim<cplx> pr = node_prim<GAS>(g, s[0], s[1], s[2], s[3]);
-        const cplx rEp = s[3] + pr.p, ruv = s[1] * pr.v;
+        const NodePrim<C> pr = node_prim<GAS>(g, s[0], s[1], s[2], s[3]);
+        const C rEp = s[3] + pr.p, ruv = s[1] * pr.v;
         double* A = sm + J::oA + (node * 4 + var) * 8;
         A[0] = s[1].im * a.inv_h;
         A[1] = (s[1] * pr.u + pr.p).im * a.inv_h;
@@ -153,7 +153,7 @@ __device__ __forceinline__ void jac_derivatives(const Fr2dArgs& a, int gi, int g
         }
         else
             sc = xf ? a.scale_x : a.scale_y;
-        cplx s[4], ro[RF_N], rn[RF_N], Fs[4];
+        C s[4], ro[RF_N], rn[RF_N], Fs[4];
         jac_load(a, base + own * 4, mine ? var : -1, s);
         jac_record<GAS>(g, s, ro);
         if (wall)
@@ -161,7 +161,7 @@ __device__ __forceinline__ void jac_derivatives(const Fr2dArgs& a, int gi, int g
             const int dir = xf ? (hi ? FRSDG_RIGHT : FRSDG_LEFT) : (hi ? FRSDG_TOP : FRSDG_BOTTOM);
             const int bi = xf ? (gj + a.row_base) * N + pos : gi * N + pos;
             const double2 xy = __ldg(reinterpret_cast<const double2*>(a.bxy[dir]) + bi);
-            cplx gh[4];
+            C gh[4];
             bc_ghost2<GAS>(a.bc[dir], dir, g, a.t, xy.x, xy.y, nx, ny, a.Lx, a.Ly, s, gh, a.exact_bc != 0);
 #pragma unroll
             for (int eq = 0; eq < 4; ++eq) s[eq] = gh[eq];
@@ -170,7 +170,7 @@ __device__ __forceinline__ void jac_derivatives(const Fr2dArgs& a, int gi, int g
             jac_load(a, (int64_t(nj) * a.Nx + ni) * ND + oth * 4, mine ? -1 : var, s);
         jac_record<GAS>(g, s, rn);
         // the low side of the face is the left argument
-        cplx L[RF_N], Rr[RF_N];
+        C L[RF_N], Rr[RF_N];
 #pragma unroll
         for (int f = 0; f < RF_N; ++f)
         {
@@ -178,12 +178,12 @@ __device__ __forceinline__ void jac_derivatives(const Fr2dArgs& a, int gi, int g
             Rr[f] = hi ? rn[f] : ro[f];
         }
         riemann_rec<RIEM>(L, Rr, nx, ny, Fs);
-        cplx fn[4] = {cplx(0.0), cplx(0.0), cplx(0.0), cplx(0.0)};
+        C fn[4] = {C(0.0), C(0.0), C(0.0), C(0.0)};
         if (mine)
         {
             // F.n of the own trace
-            const cplx rEp = ro[RF_E] + ro[RF_P];
-            const cplx ru = ro[RF_RHO] * ro[RF_U], rv = ro[RF_RHO] * ro[RF_V], ruv = ru * ro[RF_V];
+            const C rEp = ro[RF_E] + ro[RF_P];
+            const C ru = ro[RF_RHO] * ro[RF_U], rv = ro[RF_RHO] * ro[RF_V], ruv = ru * ro[RF_V];
             fn[0] = ru * nx + rv * ny;
             fn[1] = (ru * ro[RF_U] + ro[RF_P]) * nx + ruv * ny;
             fn[2] = ruv * nx + (rv * ro[RF_V] + ro[RF_P]) * ny;
@@ -255,15 +255,15 @@ __device__ __forceinline__ void jac_other(const double* sm, int slot, int rn, in
 }
 
 // All entries of `slots` blocks per element, blocks[((e * slots + s) * ND + col) * ND + row].
-template <int N, int GAS, int RIEM>
-__global__ void __launch_bounds__(kJacThreads) jac2d_blocks_kernel(const __grid_constant__ Fr2dArgs a, double* blocks,
+template <class C, int N, int GAS, int RIEM>
+__global__ void __launch_bounds__(kJacThreads, 3) jac2d_blocks_kernel(const __grid_constant__ Fr2dArgs a, double* blocks,
                                                                    int slots)
 {
     using J = Jac2D<N>;
     constexpr int NN = J::NN, ND = J::ND;
     extern __shared__ __align__(16) double sm[];
     const int gi = int(blockIdx.x) % a.Nx, gj = a.row_begin + int(blockIdx.x) / a.Nx;
-    jac_derivatives<N, GAS, RIEM>(a, gi, gj, sm);
+    jac_derivatives<C, N, GAS, RIEM>(a, gi, gj, sm);
     const int64_t mbase = (int64_t(gj + a.row_base) * a.Nx + gi) * NN;
     double* out = blocks + (int64_t(gj) * a.Nx + gi) * slots * (int64_t(ND) * ND);
     for (int q = threadIdx.x; q < slots * ND * NN; q += kJacThreads)
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kJacThreads) jac2d_blocks_kernel(const __grid_
 // warp finds the pivot by itself, and the pivot row) instead of six in shared memory.
 // 256 x 64 elements, p = 3 (n = 64), the whole Gauss-Seidel set-up: 21.9 -> 3.5 ms against
 // the coloured launch with the shared-memory elimination; p = 5 (n = 144) 286 -> 32 ms.
-template <int N, int GAS, int RIEM>
+template <class C, int N, int GAS, int RIEM>
 __global__ void __launch_bounds__(kJacThreads, Jac2D<N>::R <= 4 ? 3 : 1) jac2d_inverse_kernel(const __grid_constant__ Fr2dArgs a, float* inv,
                                                                     float4* off, unsigned long long* singular)
 {
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kJacThreads, Jac2D<N>::R <= 4 ? 3 : 1) jac2d_i
     const int gi = int(blockIdx.x) % a.Nx, gj = a.row_begin + int(blockIdx.x) / a.Nx;
     const int64_t e = int64_t(gj) * a.Nx + gi;
     const int64_t mbase = (int64_t(gj + a.row_base) * a.Nx + gi) * NN;
-    jac_derivatives<N, GAS, RIEM>(a, gi, gj, sm);
+    jac_derivatives<C, N, GAS, RIEM>(a, gi, gj, sm);
     if (off)
         for (int q = tid; q < 4 * NN; q += kJacThreads)
         {
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kJacThreads, Jac2D<N>::R <= 4 ? 3 : 1) jac2d_i
             perm[k] = br;
             pinv[br] = k;
         }
-        const double rp = 1.0 / scol[br];
+        const double rp = s_rcp(scol[br]);
         const int rq = br >> 4;
         if (ty == (br & 15))
         {
@@ -450,38 +450,38 @@ __global__ void __launch_bounds__(kJacThreads, Jac2D<N>::R <= 4 ? 3 : 1) jac2d_i
     for (int q = tid; q < ND * ND / 4; q += kJacThreads) dst[q] = reinterpret_cast<const float4*>(sout)[q];
 }
 
-template <int N, int GAS, int RIEM> cudaError_t launch_jac2d_kernel(const Fr2dArgs& a, const JacOut& o, cudaStream_t st)
+template <class C, int N, int GAS, int RIEM> cudaError_t launch_jac2d_kernel(const Fr2dArgs& a, const JacOut& o, cudaStream_t st)
 {
     using J = Jac2D<N>;
     const unsigned grid = unsigned(int64_t(a.Nx) * (a.row_end - a.row_begin));
     if (o.blocks)
     {
-        cudaError_t e = cudaFuncSetAttribute(jac2d_blocks_kernel<N, GAS, RIEM>,
+        cudaError_t e = cudaFuncSetAttribute(jac2d_blocks_kernel<C, N, GAS, RIEM>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(J::bytes));
         if (e != cudaSuccess) return e;
-        jac2d_blocks_kernel<N, GAS, RIEM><<<grid, kJacThreads, J::bytes, st>>>(a, o.blocks, o.slots);
+        jac2d_blocks_kernel<C, N, GAS, RIEM><<<grid, kJacThreads, J::bytes, st>>>(a, o.blocks, o.slots);
         return cudaGetLastError();
     }
     if constexpr (J::ND <= kMaxBlockDofs)
     {
-        cudaError_t e = cudaFuncSetAttribute(jac2d_inverse_kernel<N, GAS, RIEM>,
+        cudaError_t e = cudaFuncSetAttribute(jac2d_inverse_kernel<C, N, GAS, RIEM>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(J::inv_bytes));
         if (e != cudaSuccess) return e;
-        jac2d_inverse_kernel<N, GAS, RIEM>
+        jac2d_inverse_kernel<C, N, GAS, RIEM>
             <<<grid, kJacThreads, J::inv_bytes, st>>>(a, o.inv, reinterpret_cast<float4*>(o.off), o.singular);
         return cudaGetLastError();
     }
     return cudaErrorInvalidValue;
 }
 
-template <int N> cudaError_t launch_jac2d(int gas, int riem, const Fr2dArgs& a, const JacOut& o, cudaStream_t s)
+template <class C, int N> cudaError_t launch_jac2d(int gas, int riem, const Fr2dArgs& a, const JacOut& o, cudaStream_t s)
 {
     switch (gas * 2 + riem)
     {
-        case 0: return launch_jac2d_kernel<N, 0, 0>(a, o, s);
-        case 1: return launch_jac2d_kernel<N, 0, 1>(a, o, s);
-        case 2: return launch_jac2d_kernel<N, 1, 0>(a, o, s);
-        case 3: return launch_jac2d_kernel<N, 1, 1>(a, o, s);
+        case 0: return launch_jac2d_kernel<C, N, 0, 0>(a, o, s);
+        case 1: return launch_jac2d_kernel<C, N, 0, 1>(a, o, s);
+        case 2: return launch_jac2d_kernel<C, N, 1, 0>(a, o, s);
+        case 3: return launch_jac2d_kernel<C, N, 1, 1>(a, o, s);
         default: return cudaErrorInvalidValue;
     }
 }

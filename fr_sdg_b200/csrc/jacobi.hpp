@@ -24,7 +24,7 @@ struct JacOut
     unsigned long long* singular;
 };
 struct Fr2dArgs;
-template <int N> cudaError_t launch_jac2d(int gas, int riem, const Fr2dArgs& a, const JacOut& o, cudaStream_t s);
+template <class C, int N> cudaError_t launch_jac2d(int gas, int riem, const Fr2dArgs& a, const JacOut& o, cudaStream_t s);
 // FP32 values of `off` per element: four neighbours, ND rows, four columns each
 inline int64_t offdiag_floats(int nd) { return int64_t(16) * nd; }
 // z = M^-1 r on an Nx x Ny element grid with n points per direction: the element blocks'

@@ -21,7 +21,7 @@ namespace
 // 302 MB read: 150 -> 75 us).
 constexpr int kPPElems = 32;
 
-template <int N> __global__ void __launch_bounds__(256) pp_limit2d_kernel(const PPArgs a)
+template <int N> __global__ void __launch_bounds__(256, 3) pp_limit2d_kernel(const __grid_constant__ PPArgs a)
 {
     constexpr int NQ = N * N;
     __shared__ int flag[kPPElems];
@@ -52,7 +52,7 @@ template <int N> __global__ void __launch_bounds__(256) pp_limit2d_kernel(const 
     }
 }
 
-template <int N> __global__ void __launch_bounds__(256) pp_batch_kernel(const PPBatchArgs b)
+template <int N> __global__ void __launch_bounds__(256) pp_batch_kernel(const __grid_constant__ PPBatchArgs b)
 {
     constexpr int NQ = N * N;
     const int64_t g = int64_t(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32;
@@ -104,37 +104,10 @@ __global__ void batch_clock_kernel(BatchClock* clock, int count, int* active_cou
     }
 }
 
-template <int N> __global__ void __launch_bounds__(128) pp_limit1d_kernel(const PPArgs a)
+template <int N> __global__ void __launch_bounds__(128) pp_limit1d_kernel(const __grid_constant__ PPArgs a)
 {
     const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= a.nelem) return;
-    double* u = a.U + e * (3 * N);
-    double wsum = 0.0, ub[3] = {0.0, 0.0, 0.0};
-    for (int q = 0; q < N; ++q)
-    {
-        wsum += a.w[q];
-        for (int c = 0; c < 3; ++c) ub[c] += a.w[q] * u[c * N + q];
-    }
-    for (int c = 0; c < 3; ++c) ub[c] /= wsum;
-    const double pb = pp_pressure<3>(a, ub);
-    if (!(ub[0] > 0.0) || !(pb > 0.0)) return;
-    const double eps = fmin(a.eps0, fmin(ub[0], pb));
-    double rmin = u[0];
-    for (int q = 1; q < N; ++q) rmin = fmin(rmin, u[q]);
-    if (rmin < eps)
-    {
-        const double th1 = (ub[0] - eps) / (ub[0] - rmin);
-        for (int q = 0; q < N; ++q) u[q] = ub[0] + th1 * (u[q] - ub[0]);
-    }
-    double th2 = 1.0;
-    for (int q = 0; q < N; ++q)
-    {
-        const double uq[3] = {u[q], u[N + q], u[2 * N + q]};
-        if (!(pp_pressure<3>(a, uq) >= eps)) th2 = fmin(th2, pp_segment_root<3>(a, ub, uq, eps));
-    }
-    if (th2 < 1.0)
-        for (int q = 0; q < N; ++q)
-            for (int c = 0; c < 3; ++c) u[c * N + q] = ub[c] + th2 * (u[c * N + q] - ub[c]);
+    if (e < a.nelem) pp_element1d<N>(a, a.U + e * (3 * N));
 }
 
 template <int N> cudaError_t launch_pp_batch_n(const PPBatchArgs& b, cudaStream_t s)

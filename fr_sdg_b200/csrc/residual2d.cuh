@@ -187,28 +187,31 @@ template <> struct NodeLoader<float>
     }
 };
 
-template <> struct NodeLoader<cplx>
+// the complex-step point u + i h v (dual: h = 1)
+template <class C> struct ComplexLoader
 {
-    __device__ static void load(const Fr2dArgs& a, int64_t off, cplx s[4])
+    __device__ static void load(const Fr2dArgs& a, int64_t off, C s[4])
     {
         const double2 x0 = __ldg(reinterpret_cast<const double2*>(a.U + off));
         const double2 x1 = __ldg(reinterpret_cast<const double2*>(a.U + off + 2));
         const double2 v0 = __ldg(reinterpret_cast<const double2*>(a.W + off));
         const double2 v1 = __ldg(reinterpret_cast<const double2*>(a.W + off + 2));
-        s[0] = cplx(x0.x, v0.x * a.h);
-        s[1] = cplx(x0.y, v0.y * a.h);
-        s[2] = cplx(x1.x, v1.x * a.h);
-        s[3] = cplx(x1.y, v1.y * a.h);
+        s[0] = C(x0.x, v0.x * a.h);
+        s[1] = C(x0.y, v0.y * a.h);
+        s[2] = C(x1.x, v1.x * a.h);
+        s[3] = C(x1.y, v1.y * a.h);
         if (a.cond_sys)
         {
-            const cplx rho  = s_exp(s[0]);
-            const cplx ssq  = (cplx(0.0) + s[1] * s[1]) + s[2] * s[2];
-            const cplx rhoE = rho * (s_exp(s[3]) + 0.5 * ssq);
-            const cplx u = s[1], v = s[2];
+            const C rho  = s_exp(s[0]);
+            const C ssq  = (C(0.0) + s[1] * s[1]) + s[2] * s[2];
+            const C rhoE = rho * (s_exp(s[3]) + 0.5 * ssq);
+            const C u = s[1], v = s[2];
             s[0] = rho; s[1] = rho * u; s[2] = rho * v; s[3] = rhoE;
         }
     }
 };
+template <> struct NodeLoader<cplx> : ComplexLoader<cplx> {};
+template <> struct NodeLoader<dual> : ComplexLoader<dual> {};
 
 template <int GAS, class S>
 __device__ __forceinline__ void make_record(const GasParams& g, const S s[4], const NodePrim<S>& pr, S rec[RF_N])
