@@ -17,7 +17,8 @@
 // One CTA per element.  Two forms:
 //   blocks   every entry of 1 or 5 blocks per element written out (frsdg_jac_blocks,
 //            frsdg_jac_blocks5): 256 x 64 elements, p = 3, five blocks (2.7 GB) 13.95 ms
-//            with one residual per column and colour, 1.71 ms assembled;
+//            with one residual per column and colour, 1.71 ms assembled (one
+//            CTA per SM, complex), 0.77 ms with three and first-order scalars;
 //   inverse  the diagonal block assembled into registers, inverted there in FP64 and kept
 //            in FP32, and the neighbours' entries kept in FP32, nonzeros only
 //            (frsdg_pc_setup, frsdg_pc_setup_gs): bound by the elimination's FP64 work and
@@ -299,8 +300,9 @@ __global__ void __launch_bounds__(kJacThreads, 3) jac2d_blocks_kernel(const __gr
 // equation r_k, the unused row with the largest entry of column k, without moving rows; the
 // inverse is B[r_k][j] at (k, r_j).  Two barriers per step (the column, from which every
 // warp finds the pivot by itself, and the pivot row) instead of six in shared memory.
-// 256 x 64 elements, p = 3 (n = 64), the whole Gauss-Seidel set-up: 21.9 -> 3.5 ms against
-// the coloured launch with the shared-memory elimination; p = 5 (n = 144) 286 -> 32 ms.
+// 256 x 64 elements, p = 3 (n = 64), the whole Gauss-Seidel set-up: 21.9 -> 2.0 ms against
+// the coloured launch with the shared-memory elimination; p = 5 (n = 144) 286 -> 19 ms (3.3 and
+// 31 ms with run-time column selects and ten shuffles per pivot).
 template <class C, int N, int GAS, int RIEM>
 __global__ void __launch_bounds__(kJacThreads, Jac2D<N>::R <= 4 ? 3 : 1) jac2d_inverse_kernel(const __grid_constant__ Fr2dArgs a, float* inv,
                                                                     float4* off, unsigned long long* singular)
@@ -345,91 +347,103 @@ __global__ void __launch_bounds__(kJacThreads, Jac2D<N>::R <= 4 ? 3 : 1) jac2d_i
         }
     unsigned used = 0;  // bit t: row lane + 32 t is exchanged already
     bool bad = false;
+    // steps k = 16 kq + kk: the column's place among the thread's R is known at compile time
+    auto steps = [&](auto kq_tag) {
+        constexpr int kq = decltype(kq_tag)::value;
+        constexpr int kend = ND - kq * 16 < 16 ? ND - kq * 16 : 16;
+        if (bad) return;
 #pragma unroll 1
-    for (int k = 0; k < ND; ++k)
-    {
-        const int kq = k >> 4;
-        if (tx == (k & 15))
+        for (int kk = 0; kk < kend; ++kk)
         {
+            const int k = kq * 16 + kk;
+            if (tx == kk)
+            {
+                // hand the column out; its entries restart from the exchange's 0
 #pragma unroll
-            for (int q = 0; q < R; ++q)
-                if (q == kq)
+                for (int p = 0; p < R; ++p)
                 {
+                    if (ty + 16 * p < ND) scol[ty + 16 * p] = B[p][kq];
+                    B[p][kq] = 0.0;
+                }
+            }
+            __syncthreads();
+            // pivot: the unused row with the largest |column entry|, compared by the leading 32
+            // bits (the lowest row among equals), two warp reductions in every warp
+            unsigned best = 0;
+            int br = ND;
+#pragma unroll
+            for (int t = 0; t < (ND + 31) / 32; ++t)
+            {
+                const int i = lane + 32 * t;
+                if (i < ND && !((used >> t) & 1u))
+                {
+                    // NaN entries are never chosen; a subnormal one counts as zero
+                    const unsigned v = static_cast<unsigned>(__double2hiint(scol[i])) & 0x7fffffffu;
+                    if (v > best && v <= 0x7ff00000u) { best = v; br = i; }
+                }
+            }
+            const unsigned top = __reduce_max_sync(0xffffffffu, best);
+            br = __reduce_min_sync(0xffffffffu, best == top ? br : ND);
+            if (top < 0x00100000u)
+            {
+                bad = true;  // uniform over the CTA: every warp reads the same column
+                break;
+            }
+            if ((br & 31) == lane) used |= 1u << (br >> 5);
+            if (tid == 0)
+            {
+                perm[k] = br;
+                pinv[br] = k;
+            }
+            double f[R];
+#pragma unroll
+            for (int p = 0; p < R; ++p) f[p] = ty + 16 * p < ND ? scol[ty + 16 * p] : 0.0;
+            if (ty == (br & 15))
+            {
+                // the pivot row, scaled (selects: branches on p would index B at run time)
+                const double rp = s_rcp(scol[br]);
+                const int rq = br >> 4;
+                double fac[R];
+#pragma unroll
+                for (int p = 0; p < R; ++p)
+                {
+                    fac[p] = p == rq ? rp : 1.0;
+                    f[p] = p == rq ? 0.0 : f[p];
+                    B[p][kq] = tx == kk && p == rq ? 1.0 : B[p][kq];
+                }
+#pragma unroll
+                for (int q = 0; q < R; ++q)
+                {
+                    double v = 0.0;
 #pragma unroll
                     for (int p = 0; p < R; ++p)
-                        if (ty + 16 * p < ND) scol[ty + 16 * p] = B[p][q];
-                }
-        }
-        __syncthreads();
-        // pivot: the largest |column entry| among the unused rows, the lowest row among equals
-        double best = -1.0;
-        int br = ND;
-#pragma unroll
-        for (int t = 0; t < (ND + 31) / 32; ++t)
-        {
-            const int i = lane + 32 * t;
-            if (i < ND && !((used >> t) & 1u))
-            {
-                const double v = fabs(scol[i]);
-                if (v > best) { best = v; br = i; }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, br, o);
-            if (ov > best || (ov == best && oi < br)) { best = ov; br = oi; }
-        }
-        if (!(best > 0.0))
-        {
-            bad = true;  // uniform over the CTA: every warp reads the same column
-            break;
-        }
-        if ((br & 31) == lane) used |= 1u << (br >> 5);
-        if (tid == 0)
-        {
-            perm[k] = br;
-            pinv[br] = k;
-        }
-        const double rp = s_rcp(scol[br]);
-        const int rq = br >> 4;
-        if (ty == (br & 15))
-        {
-#pragma unroll
-            for (int p = 0; p < R; ++p)
-                if (p == rq)
-                {
-#pragma unroll
-                    for (int q = 0; q < R; ++q)
                     {
-                        const int j = tx + 16 * q;
-                        B[p][q] = (j == k ? 1.0 : B[p][q]) * rp;
-                        if (j < ND) srow[j] = B[p][q];
+                        B[p][q] *= fac[p];
+                        v = p == rq ? B[p][q] : v;
                     }
+                    if (tx + 16 * q < ND) srow[tx + 16 * q] = v;
                 }
-        }
-        double f[R];
+            }
+            __syncthreads();
 #pragma unroll
-        for (int p = 0; p < R; ++p)
-        {
-            const int i = ty + 16 * p;
-            f[p] = i < ND && i != br ? scol[i] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < R; ++q)
-        {
-            const int j = tx + 16 * q;
-            const double rj = j < ND ? srow[j] : 0.0;
-#pragma unroll
-            for (int p = 0; p < R; ++p)
+            for (int q = 0; q < R; ++q)
             {
-                const double b = (j == k && ty + 16 * p != br) ? 0.0 : B[p][q];
-                B[p][q] = fma(-f[p], rj, b);
+                const double rj = tx + 16 * q < ND ? srow[tx + 16 * q] : 0.0;
+#pragma unroll
+                for (int p = 0; p < R; ++p) B[p][q] = fma(-f[p], rj, B[p][q]);
             }
         }
-    }
+    };
+    static_assert(R <= 9, "register tile");
+    steps(std::integral_constant<int, 0>{});
+    if constexpr (R > 1) steps(std::integral_constant<int, 1>{});
+    if constexpr (R > 2) steps(std::integral_constant<int, 2>{});
+    if constexpr (R > 3) steps(std::integral_constant<int, 3>{});
+    if constexpr (R > 4) steps(std::integral_constant<int, 4>{});
+    if constexpr (R > 5) steps(std::integral_constant<int, 5>{});
+    if constexpr (R > 6) steps(std::integral_constant<int, 6>{});
+    if constexpr (R > 7) steps(std::integral_constant<int, 7>{});
+    if constexpr (R > 8) steps(std::integral_constant<int, 8>{});
     if (bad)
     {
         // zero pivot: the inverse is left unwritten; the caller reports the failure
