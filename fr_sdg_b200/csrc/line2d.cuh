@@ -43,8 +43,11 @@ enum : unsigned
 
 constexpr int kSMs = 148;  // B200: residencies and prefetch distances are counted in its SMs
 
-template <int N, int GEO, int VAR = 0> struct Line2D
+// The FP32 residual (S = float) keeps the four equations of a node in one 16-byte plane and a
+// record in a float4 and a float2.
+template <int N, int GEO, int VAR = 0, class S = double> struct Line2D
 {
+    static constexpr bool F32 = sizeof(S) == 4;
     static constexpr int NN = N * N, ND = 4 * NN;
     // VAR 0: the tuned tile; 1: half its rows (a candidate of the batch autotuner); 2: a
     // 4 x 4 tile with a warp per 32 face points, one round of the face pass instead of
@@ -67,7 +70,8 @@ template <int N, int GEO, int VAR = 0> struct Line2D
     static constexpr int ES = N == 2 ? 6 : N == 3 ? 15 : N == 4 ? 20 : N == 5 ? 37 : N <= 9 ? N * RS : 114;
     static constexpr int ROT = N == 5 ? 2 : 0;             // row of thread m of element e: (m + ROT e) mod N
     static constexpr int PLANE = TE * ES;
-    static constexpr int NPLANE = GEO == GEO_CURVED ? 4 : 2;
+    static constexpr int NP = F32 ? 1 : 2;                 // planes of a flux
+    static constexpr int NPLANE = GEO == GEO_CURVED ? 2 * NP : NP;
     // Face records, three planes (rho, rho E | u, v | p, c): the four face lines of each
     // element (corner nodes twice), then the halo traces.  A record is read by the one face
     // point of its line and then holds the jump of that side in its first two planes.
@@ -77,7 +81,7 @@ template <int N, int GEO, int VAR = 0> struct Line2D
     static constexpr int HXL = TE * DS, HXR = HXL + TY * N, HYB = HXR + TY * N, HYT = HYB + TX * N;
     static constexpr int RPL = TE * DS + NHALO;
     static constexpr size_t oRec = size_t(NPLANE) * PLANE * 16;
-    static constexpr size_t bytes = oRec + size_t(3) * RPL * 16;
+    static constexpr size_t bytes = oRec + size_t(RPL) * (F32 ? 24 : 48);
     static_assert(RPL < 4096, "records fit the packed face points");
     __host__ __device__ static constexpr unsigned face_point(bool xf, int t, int txe, int tye)
     {
@@ -92,9 +96,11 @@ template <int N, int GEO, int VAR = 0> struct Line2D
     }
     // Co-resident CTAs: what shared memory admits, at most 16 warps at n <= 4 and in the small
     // variant (128 registers), 15 at n = 5, 12 above (168 registers: at n = 6, 15 warps with
-    // narrower strides spill, 0.80 against 0.73 ms on the 1024^2 blast; nine warps are as fast)
+    // narrower strides spill, 0.80 against 0.73 ms on the 1024^2 blast; nine warps are as fast);
+    // FP32 16 (512^2 blast, p = 3, 4, 5: 0.134, 0.201, 0.217 ms with the face tiles, 0.059,
+    // 0.094, 0.117 here; 12 to 24 warps within 8 %)
     static constexpr int CTAS_SM = int((227 * 1024) / (bytes + 1024));
-    static constexpr int WARPS = VAR == 2 || N <= 4 ? 16 : N == 5 ? 15 : 12;
+    static constexpr int WARPS = F32 || VAR == 2 || N <= 4 ? 16 : N == 5 ? 15 : 12;
     static constexpr int CTAS_W = WARPS / NW > 0 ? WARPS / NW : 1;
     static constexpr int CTAS = CTAS_SM < CTAS_W ? (CTAS_SM > 0 ? CTAS_SM : 1) : CTAS_W;
 };
@@ -121,6 +127,11 @@ __device__ __forceinline__ void load_node(const Fr2dArgs& a, int64_t off, double
     const double2 x0 = __ldg(reinterpret_cast<const double2*>(a.U + off));
     const double2 x1 = __ldg(reinterpret_cast<const double2*>(a.U + off + 2));
     s[0] = x0.x; s[1] = x0.y; s[2] = x1.x; s[3] = x1.y;
+}
+__device__ __forceinline__ void load_node(const Fr2dArgs& a, int64_t off, float s[4])
+{
+    const float4 x = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.U) + off));
+    s[0] = x.x; s[1] = x.y; s[2] = x.z; s[3] = x.w;
 }
 // 32-byte accesses of a node (p 32-byte aligned)
 __device__ __forceinline__ void load_node32(const double* p, double s[4])
@@ -292,462 +303,11 @@ __device__ __forceinline__ void line_epilogue(const Fr2dArgs& a, const Ops& ops,
     if (want_amax && tid == 0 && s_amax) atomicMax(P.amax, s_amax);
 }
 
-// A tile's inputs of one thread: its column and its halo node (record -1: none).
-template <int N> struct LineIn
+// The requested output form of an FP64 column (Mode), E its residual.
+template <class T, int N, int GAS, bool POST>
+__device__ __forceinline__ void line_output(const Fr2dArgs& a, const Ops& ops, bool own, int e, int m, int64_t ebase,
+                                            int i0, int j0, int txe, int tye, double (&E)[4][N], double2* sF)
 {
-    double u[N][4];
-    double hs[4];
-    int    hrec;
-};
-
-// Halo node q of tile (bx, by): its offset in U and its record, or -1.
-template <class T, int N>
-__device__ __forceinline__ int line_halo(const Fr2dArgs& a, int bx, int by, int q, int64_t& off)
-{
-    constexpr int TX = T::TX, TY = T::TY, ND = T::ND;
-    const int Nx = a.Nx, Ny = a.Ny;
-    const int i0 = bx * TX, j0 = by * TY + a.row_begin;
-    const int txe = min(TX, Nx - i0), tye = min(TY, a.row_end - j0);
-    int ge_i, ge_j, node, r;
-    bool ok;
-    if (q < 2 * TY * N)
-    {
-        const int side = q / (TY * N), y = (q % (TY * N)) / N, p = q % N;
-        ok = y < tye;
-        ge_j = j0 + y;
-        ge_i = side == 0 ? i0 - 1 : i0 + txe;
-        if (ge_i < 0 || ge_i >= Nx)
-        {
-            ok = ok && a.per_x;
-            ge_i = ge_i < 0 ? ge_i + Nx : ge_i - Nx;
-        }
-        node = p * N + (side == 0 ? N - 1 : 0);
-        r = T::HXL + q;
-    }
-    else
-    {
-        const int qq = q - 2 * TY * N;
-        const int side = qq / (TX * N), x = (qq % (TX * N)) / N, p = qq % N;
-        ok = x < txe;
-        ge_i = i0 + x;
-        ge_j = side == 0 ? j0 - 1 : j0 + tye;
-        if (ge_j < 0 || ge_j >= Ny)
-        {
-            ok = ok && a.per_y;
-            ge_j = ge_j < 0 ? ge_j + Ny : ge_j - Ny;
-        }
-        node = side == 0 ? (N - 1) * N + p : p;
-        r = T::HYB + qq;
-    }
-    off = (int64_t(ge_j) * Nx + ge_i) * ND + node * 4;
-    return ok ? r : -1;
-}
-
-// The loads of a tile's inputs, all in flight at once (as stored; cond_sys maps them later).
-template <class T, int N>
-__device__ __forceinline__ void line_load(const Fr2dArgs& a, int bx, int by, LineIn<N>& in)
-{
-    constexpr int TX = T::TX, TY = T::TY, ND = T::ND;
-    const int tid = threadIdx.x;
-    const int m = tid % N, e = tid / N, i = bx * TX + e % TX, j = by * TY + a.row_begin + e / TX;
-    int64_t hoff = 0;
-    in.hrec = tid < T::NHALO ? line_halo<T, N>(a, bx, by, tid, hoff) : -1;
-    const bool mine = tid < T::NT && i < a.Nx && j < a.row_end;
-    const int64_t base = (int64_t(j) * a.Nx + i) * ND + m * 4;
-    if ((reinterpret_cast<uintptr_t>(a.U) & 31) == 0)
-    {
-        if (in.hrec >= 0) load_node32(a.U + hoff, in.hs);
-        if (!mine) return;
-#pragma unroll
-        for (int l = 0; l < N; ++l) load_node32(a.U + base + l * N * 4, in.u[l]);
-    }
-    else
-    {
-        if (in.hrec >= 0) load_node(a, hoff, in.hs);
-        if (!mine) return;
-#pragma unroll
-        for (int l = 0; l < N; ++l) load_node(a, base + l * N * 4, in.u[l]);
-    }
-}
-
-// One tile (bx, by); smem: T::bytes, 16-byte aligned.  Consecutive tiles of a CTA need no
-// barrier in between: what the output pass reads of shared memory, the same thread
-// overwrites next.
-template <int N, int GAS, int RIEM, int GEO, int VAR, bool POST>
-__device__ __forceinline__ void fr2d_line_tile(const Fr2dArgs& a, const Ops& ops, int bx, int by, unsigned char* smem)
-{
-    using T = Line2D<N, GEO, VAR>;
-    constexpr int TX = T::TX, TY = T::TY, TE = T::TE, NN = T::NN, ND = T::ND, BT = T::BT;
-    double2* sF = reinterpret_cast<double2*>(smem);                    // [plane][e ES + l RS + k]
-    double2* sG = sF + 2 * T::PLANE;                                   // curved only
-    double2* sR = reinterpret_cast<double2*>(smem + T::oRec);          // records [plane][e DS + side N + pos], halo
-    LineIn<N> in;
-    line_load<T, N>(a, bx, by, in);
-    const int tid = threadIdx.x;
-    const int Nx = a.Nx, Ny = a.Ny;
-    const int i0 = bx * TX, j0 = by * TY + a.row_begin;
-    const int txe = min(TX, Nx - i0), tye = min(TY, a.row_end - j0);
-    const GasParams g = a.gas;
-    const bool line = tid < T::NT;
-    const int m = tid % N, e = line ? tid / N : 0, tx = e % TX, ty = e / TX;  // line m of element e
-    const bool own = line && tx < txe && ty < tye;
-    const int64_t ebase = (int64_t(j0 + ty) * Nx + (i0 + tx)) * ND;
-    const int64_t mbase = (int64_t(j0 + ty + a.row_base) * Nx + (i0 + tx)) * NN;
-
-    // operands of the output pass: their lines into L2 first (hints)
-    if (a.mode == MODE_STAGE || a.mode == MODE_IFUNC)
-    {
-        constexpr int LROW = (TX * ND * int(sizeof(double)) + 127) / 128;
-        const int lrow = (txe * ND * int(sizeof(double)) + 127) / 128;
-        const double* b0 = a.mode == MODE_STAGE ? a.st.A : a.W;
-        const double* b1 = a.mode == MODE_STAGE ? a.st.B : nullptr;
-        for (int q = tid; q < 2 * TY * LROW; q += BT)
-        {
-            const int which = q / (TY * LROW), r = q % (TY * LROW), y = r / LROW, ln = r % LROW;
-            const double* base = which ? b1 : b0;
-            if (base && base != a.U && y < tye && ln < lrow)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (int64_t(j0 + y) * Nx + i0) * ND + ln * 16));
-        }
-    }
-
-    // A face record.  Affine meshes keep the velocities in the face's frame (normal,
-    // tangential: (u, v) on x-faces, (v, -u) on y-faces), so that one copy of the face
-    // pass serves both directions; jumps are left in that frame too.
-    constexpr bool AFF = GEO == GEO_AFFINE;
-    // face point of this lane in chunk c, loaded a round ahead
-    const bool full = txe == TX && tye == TY;
-    auto face_word = [&](int c) -> unsigned {
-        if (c >= T::CX + T::CY) return 0u;
-        return full ? __ldg(&kFaceTable<T>.v[c * 32 + (tid & 31)])
-                    : T::face_point(c < T::CX, (c < T::CX ? c : c - T::CX) * 32 + (tid & 31), txe, tye);
-    };
-    unsigned next_fp = face_word(tid / 32);
-    auto put_record = [&](int r, bool yface, const double s[4], const NodePrim<double>& pr, double c) {
-        sR[r] = make_double2(s[0], s[3]);
-        sR[T::RPL + r] = AFF && yface ? make_double2(pr.v, -pr.u) : make_double2(pr.u, pr.v);
-        sR[2 * T::RPL + r] = make_double2(pr.p, c);
-    };
-    auto halo_node = [&](int r, const double s[4], const auto& mth) {
-        const NodePrim<double> pr = node_prim<GAS>(g, s[0], s[1], s[2], s[3], mth);
-        put_record(r, r >= T::HYB, s, pr, node_sound_speed<GAS>(g, pr, mth));
-    };
-    // one node of the column: fluxes to shared memory (F; curved also G) and g4 / f4, records
-    auto column_node = [&](int l, const double s[4], double f4[4], double g4[4], const auto& mth) {
-        const NodePrim<double> pr = node_prim<GAS>(g, s[0], s[1], s[2], s[3], mth);
-        // (every node's sound speed: a branch on boundary nodes diverges in every warp)
-        const double c = node_sound_speed<GAS>(g, pr, mth);
-        const double rEp = s[3] + pr.p, ruv = s[1] * pr.v;
-        f4[0] = s[1];
-        f4[1] = s[1] * pr.u + pr.p;
-        f4[2] = ruv;
-        f4[3] = pr.u * rEp;
-        g4[0] = s[2];
-        g4[1] = ruv;
-        g4[2] = s[2] * pr.v + pr.p;
-        g4[3] = pr.v * rEp;
-        const int at = e * T::ES + l * T::RS + m;
-        sF[at] = make_double2(f4[0], f4[1]);
-        sF[T::PLANE + at] = make_double2(f4[2], f4[3]);
-        if constexpr (GEO == GEO_CURVED)
-        {
-            sG[at] = make_double2(g4[0], g4[1]);
-            sG[T::PLANE + at] = make_double2(g4[2], g4[3]);
-        }
-        if (m == 0 || m == N - 1) put_record(e * T::DS + (m == 0 ? 0 : T::oR) + l, false, s, pr, c);
-        if (l == 0 || l == N - 1) put_record(e * T::DS + (l == 0 ? T::oB : T::oT) + m, true, s, pr, c);
-    };
-
-    // ---- column pass
-    double E[4][N];  // eta part of the column's residual
-    {
-        double G[4][GEO == GEO_CURVED ? 1 : N];  // curved: both fluxes come back from shared memory
-        if (own)
-        {
-            unsigned bad = 0;
-            if (a.cond_sys)
-            {
-#pragma unroll
-                for (int l = 0; l < N; ++l) to_conservative(a, in.u[l]);
-            }
-#pragma unroll
-            for (int l = 0; l < N; ++l)
-            {
-                double f4[4], g4[4];
-                const double* s = in.u[l];
-                column_node(l, s, f4, g4, MathDeferred{bad});
-#pragma unroll
-                for (int eq = 0; eq < 4; ++eq)
-                {
-                    if constexpr (AFF) G[eq][l] = g4[eq];
-                }
-            }
-            if (bad)
-            {
-                // a reciprocal or square root met an input outside the fast range: the whole
-                // column again with the checked functions, the densities counted
-#pragma unroll 1
-                for (int l = 0; l < N; ++l)
-                {
-                    double s[4], f4[4], g4[4];
-                    load_node(a, ebase + (l * N + m) * 4, s);
-                    to_conservative(a, s);
-                    if (!density_ok(s[0]) && a.bad) atomicAdd(a.bad, 1ull);
-                    column_node(l, s, f4, g4, MathChecked{});
-                    if constexpr (AFF)
-                    {
-#pragma unroll
-                        for (int q = 0; q < N; ++q)
-                            if (q == l)
-                            {
-#pragma unroll
-                                for (int eq = 0; eq < 4; ++eq) G[eq][q] = g4[eq];
-                            }
-                    }
-                }
-            }
-        }
-        for (int q = tid; q < T::NHALO; q += BT)
-        {
-            if (q != tid)
-            {
-                int64_t hoff;
-                in.hrec = line_halo<T, N>(a, bx, by, q, hoff);
-                if (in.hrec >= 0) load_node(a, hoff, in.hs);
-            }
-            if (in.hrec < 0) continue;
-            to_conservative(a, in.hs);
-            unsigned bad = 0;
-            halo_node(in.hrec, in.hs, MathDeferred{bad});
-            if (bad) halo_node(in.hrec, in.hs, MathChecked{});
-        }
-        if (own)
-        {
-            // eta-derivative of the column (curved: of F too, with the node's metrics)
-            if constexpr (GEO == GEO_CURVED)
-            {
-                const double* mt = a.metrics + (mbase + m) * 4 + 2;
-                const int at = e * T::ES + m;
-#pragma unroll
-                for (int pl = 0; pl < 2; ++pl)
-                {
-                    double2 f[N], h[N];
-#pragma unroll
-                    for (int q = 0; q < N; ++q)
-                    {
-                        f[q] = sF[pl * T::PLANE + at + q * T::RS];
-                        h[q] = sG[pl * T::PLANE + at + q * T::RS];
-                    }
-#pragma unroll
-                    for (int l = 0; l < N; ++l)
-                    {
-                        const double2 me = __ldg(reinterpret_cast<const double2*>(mt + l * N * 4));
-                        double f0 = 0.0, f1 = 0.0, h0 = 0.0, h1 = 0.0;
-#pragma unroll
-                        for (int q = 0; q < N; ++q)
-                        {
-                            f0 = f0 + ops.D[l * N + q] * f[q].x;
-                            f1 = f1 + ops.D[l * N + q] * f[q].y;
-                            h0 = h0 + ops.D[l * N + q] * h[q].x;
-                            h1 = h1 + ops.D[l * N + q] * h[q].y;
-                        }
-                        E[2 * pl][l] = me.x * f0 + me.y * h0;
-                        E[2 * pl + 1][l] = me.x * f1 + me.y * h1;
-                    }
-                }
-            }
-            else
-            {
-#pragma unroll
-                for (int eq = 0; eq < 4; ++eq)
-#pragma unroll
-                    for (int l = 0; l < N; ++l)
-                    {
-                        double dG = 0.0;
-#pragma unroll
-                        for (int q = 0; q < N; ++q) dG = dG + ops.D[l * N + q] * G[eq][q];
-                        E[eq][l] = dG;
-                    }
-            }
-        }
-    }
-    __syncthreads();
-
-    // ---- face pass: x-faces on the first chunks of 32 points, y-faces on the others
-    {
-        const bool lowx = !a.per_x && i0 == 0, highx = !a.per_x && i0 + txe == Nx;
-        const bool lowy = !a.per_y && j0 == 0, highy = !a.per_y && j0 + tye == Ny;
-#pragma unroll 1
-        for (int c = tid / 32; c < T::CX + T::CY; c += T::NW)
-        {
-            const bool XF = c < T::CX;  // uniform across the warp
-            const unsigned fp = next_fp;
-            next_fp = face_word(c + T::NW);
-            if (!(fp & FP_ANY)) continue;
-            const int rM = fp & 0xfffu, rP = (fp >> 12) & 0xfffu;
-            const bool inM = fp & FP_LOW, inP = fp & FP_HIGH;
-            double L[RF_N], R[RF_N];
-            auto get = [&](int q, double v[RF_N]) {
-                const double2 x = sR[q], y = sR[T::RPL + q], z = sR[2 * T::RPL + q];
-                v[RF_RHO] = x.x; v[RF_E] = x.y; v[RF_U] = y.x; v[RF_V] = y.y; v[RF_P] = z.x; v[RF_C] = z.y;
-            };
-            get(rM, L);
-            get(rP, R);
-            // element and position of an own side, the low one if there is
-            const int sideM = XF ? T::oR : T::oT, sideP = XF ? 0 : T::oB;
-            auto pos_of = [&](int& ei) {
-                ei = (inM ? rM : rP) / T::DS;
-                return (inM ? rM - sideM : rP - sideP) - ei * T::DS;
-            };
-            double nx = XF ? 1.0 : 0.0, ny = XF ? 0.0 : 1.0;
-            if constexpr (GEO == GEO_CURVED)
-            {
-                int ei;
-                const int pos = pos_of(ei), up = inM ? 1 : 0;
-                const int gI = i0 + ei % TX + (XF ? up : 0), gJ = j0 + ei / TX + (XF ? 0 : up);
-                const double2 nn = XF ? __ldg(reinterpret_cast<const double2*>(a.xnorm) + (int64_t(gJ + a.row_base) * (Nx + 1) + gI) * N + pos)
-                                      : __ldg(reinterpret_cast<const double2*>(a.ynorm) + (int64_t(gJ + a.row_base) * Nx + gI) * N + pos);
-                nx = nn.x;
-                ny = nn.y;
-            }
-            // physical boundary (rare): the ghost of the interior trace
-            if ((!inM && (XF ? lowx : lowy)) || (!inP && (XF ? highx : highy)))
-            {
-                int ei;
-                const int pos = pos_of(ei);
-                const int gI = i0 + ei % TX, gJ = j0 + ei / TX;
-                const int dir = XF ? (inM ? FRSDG_RIGHT : FRSDG_LEFT) : (inM ? FRSDG_TOP : FRSDG_BOTTOM);
-                const int bi = XF ? (gJ + a.row_base) * N + pos : gI * N + pos;
-                const double2 xy = __ldg(reinterpret_cast<const double2*>(a.bxy[dir]) + bi);
-                const int node = XF ? pos * N + (inM ? N - 1 : 0) : (inM ? N - 1 : 0) * N + pos;
-                const int64_t ioff = (int64_t(gJ) * Nx + gI) * ND + node * 4;
-                const Rec<double> gh = ghost_record<GAS, double>(a, dir, ioff, xy.x, xy.y, nx, ny);
-#pragma unroll
-                for (int f = 0; f < RF_N; ++f)
-                {
-                    const double q = !AFF || XF || (f != RF_U && f != RF_V) ? gh.v[f] : f == RF_U ? gh.v[RF_V] : -gh.v[RF_U];
-                    if (inM) R[f] = q;
-                    else L[f] = q;
-                }
-            }
-            constexpr int AXIS = AFF ? 0 : 2;
-            double Fs[4], FL[4], FR[4];
-            unsigned bad = 0;
-            riemann_sides<RIEM, AXIS>(L, R, nx, ny, Fs, FL, FR, MathDeferred{bad});
-            if (bad) riemann_sides<RIEM, AXIS>(L, R, nx, ny, Fs, FL, FR, MathChecked{});
-            // affine: unscaled, the scale joins the metric factor of the element
-            auto jump = [&](int q, int side, bool hi, const double Fn[4]) {
-                if constexpr (AFF)
-                {
-                    sR[q] = make_double2(Fs[0] - Fn[0], Fs[1] - Fn[1]);
-                    sR[T::RPL + q] = make_double2(Fs[2] - Fn[2], Fs[3] - Fn[3]);
-                }
-                else
-                {
-                    const int fe = q / T::DS, pos = q - fe * T::DS - side;
-                    const int node = XF ? pos * N + (hi ? N - 1 : 0) : (hi ? N - 1 : 0) * N + pos;
-                    const double* mt = a.metrics + ((int64_t(j0 + fe / TX + a.row_base) * Nx + (i0 + fe % TX)) * NN + node) * 4 + (XF ? 0 : 2);
-                    const double2 mm = __ldg(reinterpret_cast<const double2*>(mt));
-                    const double sc = sqrt(mm.x * mm.x + mm.y * mm.y);
-                    sR[q] = make_double2(sc * (Fs[0] - Fn[0]), sc * (Fs[1] - Fn[1]));
-                    sR[T::RPL + q] = make_double2(sc * (Fs[2] - Fn[2]), sc * (Fs[3] - Fn[3]));
-                }
-            };
-            if (inM) jump(rM, sideM, true, FL);
-            if (inP) jump(rP, sideP, false, FR);
-        }
-    }
-    __syncthreads();
-
-    // ---- row pass: one row of element e, in place
-    if (own)
-    {
-        const int mr = T::ROT ? (m + T::ROT * e) % N : m;
-        const int at = e * T::ES + mr * T::RS;
-#pragma unroll
-        for (int pl = 0; pl < 2; ++pl)
-        {
-            double2* f = sF + pl * T::PLANE + at;
-            double x0[N], x1[N], y0[GEO == GEO_CURVED ? N : 1], y1[GEO == GEO_CURVED ? N : 1];
-#pragma unroll
-            for (int q = 0; q < N; ++q)
-            {
-                const double2 t = f[q];
-                x0[q] = t.x;
-                x1[q] = t.y;
-                if constexpr (GEO == GEO_CURVED)
-                {
-                    const double2 u = sG[pl * T::PLANE + at + q];
-                    y0[q] = u.x;
-                    y1[q] = u.y;
-                }
-            }
-            const double2 l2 = sR[pl * T::RPL + e * T::DS + mr], r2 = sR[pl * T::RPL + e * T::DS + T::oR + mr];
-#pragma unroll
-            for (int k = 0; k < N; ++k)
-            {
-                double d0 = 0.0, d1 = 0.0;
-#pragma unroll
-                for (int q = 0; q < N; ++q)
-                {
-                    d0 = d0 + ops.D[k * N + q] * x0[q];
-                    d1 = d1 + ops.D[k * N + q] * x1[q];
-                }
-                double r0, r1;
-                if constexpr (GEO == GEO_CURVED)
-                {
-                    double h0 = 0.0, h1 = 0.0;
-#pragma unroll
-                    for (int q = 0; q < N; ++q)
-                    {
-                        h0 = h0 + ops.D[k * N + q] * y0[q];
-                        h1 = h1 + ops.D[k * N + q] * y1[q];
-                    }
-                    const double2 mx = __ldg(reinterpret_cast<const double2*>(a.metrics + (mbase + mr * N + k) * 4));
-                    r0 = ((mx.x * d0 + mx.y * h0) + l2.x * ops.dL[k]) + r2.x * ops.dR[k];
-                    r1 = ((mx.x * d1 + mx.y * h1) + l2.y * ops.dL[k]) + r2.y * ops.dR[k];
-                }
-                else
-                {
-                    // xi_x is also the scale of the jumps
-                    r0 = a.xi_x * ((d0 + l2.x * ops.dL[k]) + r2.x * ops.dR[k]);
-                    r1 = a.xi_x * ((d1 + l2.y * ops.dL[k]) + r2.y * ops.dR[k]);
-                }
-                f[k] = make_double2(r0, r1);
-            }
-        }
-    }
-    __syncthreads();
-
-    // ---- output pass: column m of element e
-    if (own)
-    {
-        const double2* d = sR + e * T::DS + m;
-        double2 b0 = d[T::oB], b1 = d[T::RPL + T::oB], t0 = d[T::oT], t1 = d[T::RPL + T::oT];
-        if constexpr (AFF)
-        {
-            // from the y-faces' frame: (d0, dn | dt, d3) to (d0, -dt | dn, d3)
-            const double bn = b0.y, tn = t0.y;
-            b0.y = -b1.x;
-            b1.x = bn;
-            t0.y = -t1.x;
-            t1.x = tn;
-        }
-#pragma unroll
-        for (int l = 0; l < N; ++l)
-        {
-            const int at = e * T::ES + l * T::RS + m;
-            const double2 x0 = sF[at], x1 = sF[T::PLANE + at];
-            const double dLl = ops.dL[l], dRl = ops.dR[l];
-            auto sum = [&](double x, double eta, double b, double t) {
-                // affine: eta_y is also the scale of the jumps
-                return AFF ? x + a.eta_y * ((eta + b * dLl) + t * dRl) : ((x + eta) + b * dLl) + t * dRl;
-            };
-            E[0][l] = sum(x0.x, E[0][l], b0.x, t0.x);
-            E[1][l] = sum(x0.y, E[1][l], b0.y, t0.y);
-            E[2][l] = sum(x1.x, E[2][l], b1.x, t1.x);
-            E[3][l] = sum(x1.y, E[3][l], b1.y, t1.y);
-        }
-    }
     double* out = static_cast<double*>(a.out) + ebase + m * 4;
     auto put = [&](int l, double v0, double v1, double v2, double v3) {
         double2* o = reinterpret_cast<double2*>(out + l * N * 4);
@@ -824,8 +384,551 @@ __device__ __forceinline__ void fr2d_line_tile(const Fr2dArgs& a, const Ops& ops
     }
 }
 
-template <int N, int GAS, int RIEM, int GEO, int VAR, bool POST>
-__global__ void __launch_bounds__((Line2D<N, GEO, VAR>::BT), (Line2D<N, GEO, VAR>::CTAS))
+// A tile's inputs of one thread: its column and its halo node (record -1: none).
+template <class S, int N> struct LineIn
+{
+    S   u[N][4];
+    S   hs[4];
+    int    hrec;
+};
+
+// Halo node q of tile (bx, by): its offset in U and its record, or -1.
+template <class T, int N>
+__device__ __forceinline__ int line_halo(const Fr2dArgs& a, int bx, int by, int q, int64_t& off)
+{
+    constexpr int TX = T::TX, TY = T::TY, ND = T::ND;
+    const int Nx = a.Nx, Ny = a.Ny;
+    const int i0 = bx * TX, j0 = by * TY + a.row_begin;
+    const int txe = min(TX, Nx - i0), tye = min(TY, a.row_end - j0);
+    int ge_i, ge_j, node, r;
+    bool ok;
+    if (q < 2 * TY * N)
+    {
+        const int side = q / (TY * N), y = (q % (TY * N)) / N, p = q % N;
+        ok = y < tye;
+        ge_j = j0 + y;
+        ge_i = side == 0 ? i0 - 1 : i0 + txe;
+        if (ge_i < 0 || ge_i >= Nx)
+        {
+            ok = ok && a.per_x;
+            ge_i = ge_i < 0 ? ge_i + Nx : ge_i - Nx;
+        }
+        node = p * N + (side == 0 ? N - 1 : 0);
+        r = T::HXL + q;
+    }
+    else
+    {
+        const int qq = q - 2 * TY * N;
+        const int side = qq / (TX * N), x = (qq % (TX * N)) / N, p = qq % N;
+        ok = x < txe;
+        ge_i = i0 + x;
+        ge_j = side == 0 ? j0 - 1 : j0 + tye;
+        if (ge_j < 0 || ge_j >= Ny)
+        {
+            ok = ok && a.per_y;
+            ge_j = ge_j < 0 ? ge_j + Ny : ge_j - Ny;
+        }
+        node = side == 0 ? (N - 1) * N + p : p;
+        r = T::HYB + qq;
+    }
+    off = (int64_t(ge_j) * Nx + ge_i) * ND + node * 4;
+    return ok ? r : -1;
+}
+
+// The loads of a tile's inputs, all in flight at once (as stored; cond_sys maps them later).
+template <class T, class S, int N>
+__device__ __forceinline__ void line_load(const Fr2dArgs& a, int bx, int by, LineIn<S, N>& in)
+{
+    constexpr int TX = T::TX, TY = T::TY, ND = T::ND;
+    const int tid = threadIdx.x;
+    const int m = tid % N, e = tid / N, i = bx * TX + e % TX, j = by * TY + a.row_begin + e / TX;
+    int64_t hoff = 0;
+    in.hrec = tid < T::NHALO ? line_halo<T, N>(a, bx, by, tid, hoff) : -1;
+    const bool mine = tid < T::NT && i < a.Nx && j < a.row_end;
+    const int64_t base = (int64_t(j) * a.Nx + i) * ND + m * 4;
+    if constexpr (!T::F32)
+    {
+        if ((reinterpret_cast<uintptr_t>(a.U) & 31) == 0)
+        {
+            if (in.hrec >= 0) load_node32(a.U + hoff, in.hs);
+            if (!mine) return;
+#pragma unroll
+            for (int l = 0; l < N; ++l) load_node32(a.U + base + l * N * 4, in.u[l]);
+            return;
+        }
+    }
+    {
+        if (in.hrec >= 0) load_node(a, hoff, in.hs);
+        if (!mine) return;
+#pragma unroll
+        for (int l = 0; l < N; ++l) load_node(a, base + l * N * 4, in.u[l]);
+    }
+}
+
+// One tile (bx, by); smem: T::bytes, 16-byte aligned.  Consecutive tiles of a CTA need no
+// barrier in between: what the output pass reads of shared memory, the same thread
+// overwrites next.  S = float: MODE_RESIDUAL on an FP32 state, FP32 output.
+template <class S, int N, int GAS, int RIEM, int GEO, int VAR, bool POST>
+__device__ __forceinline__ void fr2d_line_tile(const Fr2dArgs& a, const Ops& ops, int bx, int by, unsigned char* smem)
+{
+    using T = Line2D<N, GEO, VAR, S>;
+    using V = typename std::conditional<T::F32, float4, double2>::type;  // 16 bytes of a flux plane or a record
+    constexpr int TX = T::TX, TY = T::TY, NN = T::NN, ND = T::ND, BT = T::BT;
+    constexpr bool F32 = T::F32;
+    V* sF = reinterpret_cast<V*>(smem);                    // [plane][e ES + l RS + k]
+    V* sG = sF + T::NP * T::PLANE;                         // curved only
+    V* sR = reinterpret_cast<V*>(smem + T::oRec);          // records [plane][e DS + line + pos], halo
+    float2* sR2 = reinterpret_cast<float2*>(sR + T::RPL);  // FP32: (p, c)
+    LineIn<S, N> in;
+    line_load<T>(a, bx, by, in);
+    const int tid = threadIdx.x;
+    const int Nx = a.Nx, Ny = a.Ny;
+    const int i0 = bx * TX, j0 = by * TY + a.row_begin;
+    const int txe = min(TX, Nx - i0), tye = min(TY, a.row_end - j0);
+    const GasParams g = a.gas;
+    const bool line = tid < T::NT;
+    const int m = tid % N, e = line ? tid / N : 0, tx = e % TX, ty = e / TX;  // line m of element e
+    const bool own = line && tx < txe && ty < tye;
+    const int64_t ebase = (int64_t(j0 + ty) * Nx + (i0 + tx)) * ND;
+    const int64_t mbase = (int64_t(j0 + ty + a.row_base) * Nx + (i0 + tx)) * NN;
+
+    // operands of the output pass: their lines into L2 first (hints)
+    if (a.mode == MODE_STAGE || a.mode == MODE_IFUNC)
+    {
+        constexpr int LROW = (TX * ND * int(sizeof(double)) + 127) / 128;
+        const int lrow = (txe * ND * int(sizeof(double)) + 127) / 128;
+        const double* b0 = a.mode == MODE_STAGE ? a.st.A : a.W;
+        const double* b1 = a.mode == MODE_STAGE ? a.st.B : nullptr;
+        for (int q = tid; q < 2 * TY * LROW; q += BT)
+        {
+            const int which = q / (TY * LROW), r = q % (TY * LROW), y = r / LROW, ln = r % LROW;
+            const double* base = which ? b1 : b0;
+            if (base && base != a.U && y < tye && ln < lrow)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (int64_t(j0 + y) * Nx + i0) * ND + ln * 16));
+        }
+    }
+
+    // A face record.  Affine meshes keep the velocities in the face's frame (normal,
+    // tangential: (u, v) on x-faces, (v, -u) on y-faces), so that one copy of the face
+    // pass serves both directions; jumps are left in that frame too.
+    constexpr bool AFF = GEO == GEO_AFFINE;
+    // face point of this lane in chunk c, loaded a round ahead
+    const bool full = txe == TX && tye == TY;
+    auto face_word = [&](int c) -> unsigned {
+        if (c >= T::CX + T::CY) return 0u;
+        return full ? __ldg(&kFaceTable<T>.v[c * 32 + (tid & 31)])
+                    : T::face_point(c < T::CX, (c < T::CX ? c : c - T::CX) * 32 + (tid & 31), txe, tye);
+    };
+    unsigned next_fp = face_word(tid / 32);
+    // a node's four values into the planes of a flux
+    auto put_flux = [&](V* p, int at, const S v[4]) {
+        if constexpr (F32) p[at] = make_float4(v[0], v[1], v[2], v[3]);
+        else
+        {
+            p[at] = make_double2(v[0], v[1]);
+            p[T::PLANE + at] = make_double2(v[2], v[3]);
+        }
+    };
+    auto get_flux = [&](const V* p, int at, S v[4]) {
+        if constexpr (F32)
+        {
+            const float4 x = p[at];
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        }
+        else
+        {
+            const double2 x = p[at], y = p[T::PLANE + at];
+            v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+        }
+    };
+    // the jump of a side, in the record's place
+    auto get_jump = [&](int q, S v[4]) {
+        if constexpr (F32)
+        {
+            const float4 x = sR[q];
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        }
+        else
+        {
+            const double2 x = sR[q], y = sR[T::RPL + q];
+            v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+        }
+    };
+    auto put_record = [&](int r, bool yface, const S s[4], const NodePrim<S>& pr, S c) {
+        const S un = AFF && yface ? pr.v : pr.u, ut = AFF && yface ? -pr.u : pr.v;
+        if constexpr (F32)
+        {
+            sR[r] = make_float4(s[0], s[3], un, ut);
+            sR2[r] = make_float2(pr.p, c);
+        }
+        else
+        {
+            sR[r] = make_double2(s[0], s[3]);
+            sR[T::RPL + r] = make_double2(un, ut);
+            sR[2 * T::RPL + r] = make_double2(pr.p, c);
+        }
+    };
+    auto halo_node = [&](int r, const S s[4], const auto& mth) {
+        const NodePrim<S> pr = node_prim<GAS>(g, s[0], s[1], s[2], s[3], mth);
+        put_record(r, r >= T::HYB, s, pr, node_sound_speed<GAS>(g, pr, mth));
+    };
+    // one node of the column: fluxes to shared memory (F; curved also G) and g4, records
+    auto column_node = [&](int l, const S s[4], S g4[4], const auto& mth) {
+        const NodePrim<S> pr = node_prim<GAS>(g, s[0], s[1], s[2], s[3], mth);
+        // (every node's sound speed: a branch on boundary nodes diverges in every warp)
+        const S c = node_sound_speed<GAS>(g, pr, mth);
+        const S rEp = s[3] + pr.p, ruv = s[1] * pr.v;
+        const S f4[4] = {s[1], s[1] * pr.u + pr.p, ruv, pr.u * rEp};
+        g4[0] = s[2];
+        g4[1] = ruv;
+        g4[2] = s[2] * pr.v + pr.p;
+        g4[3] = pr.v * rEp;
+        const int at = e * T::ES + l * T::RS + m;
+        put_flux(sF, at, f4);
+        if constexpr (!AFF) put_flux(sG, at, g4);
+        if (m == 0 || m == N - 1) put_record(e * T::DS + (m == 0 ? 0 : T::oR) + l, false, s, pr, c);
+        if (l == 0 || l == N - 1) put_record(e * T::DS + (l == 0 ? T::oB : T::oT) + m, true, s, pr, c);
+    };
+
+    // ---- column pass
+    S E[4][N];  // eta part of the column's residual
+    {
+        S G[4][AFF ? N : 1];  // curved: both fluxes come back from shared memory
+        if (own)
+        {
+            unsigned bad = 0;
+            if constexpr (!F32)
+            {
+                if (a.cond_sys)
+                {
+#pragma unroll
+                    for (int l = 0; l < N; ++l) to_conservative(a, in.u[l]);
+                }
+            }
+#pragma unroll
+            for (int l = 0; l < N; ++l)
+            {
+                S g4[4];
+                column_node(l, in.u[l], g4, MathDeferred{bad});
+#pragma unroll
+                for (int eq = 0; eq < 4; ++eq)
+                    if constexpr (AFF) G[eq][l] = g4[eq];
+            }
+            if (bad)
+            {
+                // a reciprocal or square root met an input outside the fast range: the whole
+                // column again with the checked functions, the densities counted (a node
+                // without such an input has a positive finite density)
+#pragma unroll 1
+                for (int l = 0; l < N; ++l)
+                {
+                    S s[4], g4[4];
+                    load_node(a, ebase + (l * N + m) * 4, s);
+                    if constexpr (!F32) to_conservative(a, s);
+                    if (!density_ok(s[0]) && a.bad) atomicAdd(a.bad, 1ull);
+                    column_node(l, s, g4, MathChecked{});
+                    if constexpr (AFF)
+                    {
+#pragma unroll
+                        for (int q = 0; q < N; ++q)
+                            if (q == l)
+                            {
+#pragma unroll
+                                for (int eq = 0; eq < 4; ++eq) G[eq][q] = g4[eq];
+                            }
+                    }
+                }
+            }
+        }
+        for (int q = tid; q < T::NHALO; q += BT)
+        {
+            if (q != tid)
+            {
+                int64_t hoff;
+                in.hrec = line_halo<T, N>(a, bx, by, q, hoff);
+                if (in.hrec >= 0) load_node(a, hoff, in.hs);
+            }
+            if (in.hrec < 0) continue;
+            if constexpr (!F32) to_conservative(a, in.hs);
+            unsigned bad = 0;
+            halo_node(in.hrec, in.hs, MathDeferred{bad});
+            if (bad) halo_node(in.hrec, in.hs, MathChecked{});
+        }
+        if (own)
+        {
+            // eta-derivative of the column (curved: of F too, with the node's metrics; affine:
+            // unscaled)
+            if constexpr (!AFF)
+            {
+                const double* mt = a.metrics + (mbase + m) * 4 + 2;
+                const int at = e * T::ES + m;
+#pragma unroll
+                for (int pl = 0; pl < T::NP; ++pl)
+                {
+                    constexpr int W = F32 ? 4 : 2;  // equations per plane
+                    S f[W][N], h[W][N];
+#pragma unroll
+                    for (int q = 0; q < N; ++q)
+                    {
+                        const V x = sF[pl * T::PLANE + at + q * T::RS], y = sG[pl * T::PLANE + at + q * T::RS];
+                        f[0][q] = x.x; f[1][q] = x.y;
+                        h[0][q] = y.x; h[1][q] = y.y;
+                        if constexpr (F32)
+                        {
+                            f[2][q] = x.z; f[3][q] = x.w;
+                            h[2][q] = y.z; h[3][q] = y.w;
+                        }
+                    }
+#pragma unroll
+                    for (int w = 0; w < W; ++w)
+                    {
+                        center_line<S, N>(f[w]);
+                        center_line<S, N>(h[w]);
+                    }
+#pragma unroll
+                    for (int l = 0; l < N; ++l)
+                    {
+                        const double2 me = __ldg(reinterpret_cast<const double2*>(mt + l * N * 4));
+#pragma unroll
+                        for (int w = 0; w < W; ++w)
+                        {
+                            S df = S(0.0), dh = S(0.0);
+#pragma unroll
+                            for (int q = 0; q < N; ++q)
+                            {
+                                df = df + opD<S>(ops, l * N + q) * f[w][q];
+                                dh = dh + opD<S>(ops, l * N + q) * h[w][q];
+                            }
+                            E[W * pl + w][l] = S(me.x) * df + S(me.y) * dh;
+                        }
+                    }
+                }
+            }
+            else
+            {
+#pragma unroll
+                for (int eq = 0; eq < 4; ++eq)
+                {
+                    center_line<S, N>(G[eq]);
+#pragma unroll
+                    for (int l = 0; l < N; ++l)
+                    {
+                        S dG = S(0.0);
+#pragma unroll
+                        for (int q = 0; q < N; ++q) dG = dG + opD<S>(ops, l * N + q) * G[eq][q];
+                        E[eq][l] = dG;
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- face pass: x-faces on the first chunks of 32 points, y-faces on the others
+    {
+        const bool lowx = !a.per_x && i0 == 0, highx = !a.per_x && i0 + txe == Nx;
+        const bool lowy = !a.per_y && j0 == 0, highy = !a.per_y && j0 + tye == Ny;
+#pragma unroll 1
+        for (int c = tid / 32; c < T::CX + T::CY; c += T::NW)
+        {
+            const bool XF = c < T::CX;  // uniform across the warp
+            const unsigned fp = next_fp;
+            next_fp = face_word(c + T::NW);
+            if (!(fp & FP_ANY)) continue;
+            const int rM = fp & 0xfffu, rP = (fp >> 12) & 0xfffu;
+            const bool inM = fp & FP_LOW, inP = fp & FP_HIGH;
+            S L[RF_N], R[RF_N];
+            auto get = [&](int q, S v[RF_N]) {
+                if constexpr (F32)
+                {
+                    const float4 x = sR[q];
+                    const float2 z = sR2[q];
+                    v[RF_RHO] = x.x; v[RF_E] = x.y; v[RF_U] = x.z; v[RF_V] = x.w; v[RF_P] = z.x; v[RF_C] = z.y;
+                }
+                else
+                {
+                    const double2 x = sR[q], y = sR[T::RPL + q], z = sR[2 * T::RPL + q];
+                    v[RF_RHO] = x.x; v[RF_E] = x.y; v[RF_U] = y.x; v[RF_V] = y.y; v[RF_P] = z.x; v[RF_C] = z.y;
+                }
+            };
+            get(rM, L);
+            get(rP, R);
+            // element and position of an own side, the low one if there is
+            const int sideM = XF ? T::oR : T::oT, sideP = XF ? 0 : T::oB;
+            auto pos_of = [&](int& ei) {
+                ei = (inM ? rM : rP) / T::DS;
+                return (inM ? rM - sideM : rP - sideP) - ei * T::DS;
+            };
+            double nx = XF ? 1.0 : 0.0, ny = XF ? 0.0 : 1.0;
+            if constexpr (GEO == GEO_CURVED)
+            {
+                int ei;
+                const int pos = pos_of(ei), up = inM ? 1 : 0;
+                const int gI = i0 + ei % TX + (XF ? up : 0), gJ = j0 + ei / TX + (XF ? 0 : up);
+                const double2 nn = XF ? __ldg(reinterpret_cast<const double2*>(a.xnorm) + (int64_t(gJ + a.row_base) * (Nx + 1) + gI) * N + pos)
+                                      : __ldg(reinterpret_cast<const double2*>(a.ynorm) + (int64_t(gJ + a.row_base) * Nx + gI) * N + pos);
+                nx = nn.x;
+                ny = nn.y;
+            }
+            // physical boundary (rare): the ghost of the interior trace
+            if ((!inM && (XF ? lowx : lowy)) || (!inP && (XF ? highx : highy)))
+            {
+                int ei;
+                const int pos = pos_of(ei);
+                const int gI = i0 + ei % TX, gJ = j0 + ei / TX;
+                const int dir = XF ? (inM ? FRSDG_RIGHT : FRSDG_LEFT) : (inM ? FRSDG_TOP : FRSDG_BOTTOM);
+                const int bi = XF ? (gJ + a.row_base) * N + pos : gI * N + pos;
+                const double2 xy = __ldg(reinterpret_cast<const double2*>(a.bxy[dir]) + bi);
+                const int node = XF ? pos * N + (inM ? N - 1 : 0) : (inM ? N - 1 : 0) * N + pos;
+                const int64_t ioff = (int64_t(gJ) * Nx + gI) * ND + node * 4;
+                const Rec<S> gh = ghost_record<GAS, S>(a, dir, ioff, xy.x, xy.y, nx, ny);
+#pragma unroll
+                for (int f = 0; f < RF_N; ++f)
+                {
+                    const S q = !AFF || XF || (f != RF_U && f != RF_V) ? gh.v[f] : f == RF_U ? gh.v[RF_V] : -gh.v[RF_U];
+                    if (inM) R[f] = q;
+                    else L[f] = q;
+                }
+            }
+            constexpr int AXIS = AFF ? 0 : 2;
+            S Fs[4], FL[4], FR[4];
+            unsigned bad = 0;
+            riemann_sides<RIEM, AXIS, S>(L, R, S(nx), S(ny), Fs, FL, FR, MathDeferred{bad});
+            if (bad) riemann_sides<RIEM, AXIS, S>(L, R, S(nx), S(ny), Fs, FL, FR, MathChecked{});
+            // affine: unscaled, the scale joins the metric factor of the element
+            auto jump = [&](int q, int side, bool hi, const S Fn[4]) {
+                S d[4];
+#pragma unroll
+                for (int eq = 0; eq < 4; ++eq) d[eq] = Fs[eq] - Fn[eq];
+                if constexpr (!AFF)
+                {
+                    const int fe = q / T::DS, pos = q - fe * T::DS - side;
+                    const int node = XF ? pos * N + (hi ? N - 1 : 0) : (hi ? N - 1 : 0) * N + pos;
+                    const double* mt = a.metrics + ((int64_t(j0 + fe / TX + a.row_base) * Nx + (i0 + fe % TX)) * NN + node) * 4 + (XF ? 0 : 2);
+                    const double2 mm = __ldg(reinterpret_cast<const double2*>(mt));
+                    const S sc = S(sqrt(mm.x * mm.x + mm.y * mm.y));
+#pragma unroll
+                    for (int eq = 0; eq < 4; ++eq) d[eq] = sc * d[eq];
+                }
+                if constexpr (F32) sR[q] = make_float4(d[0], d[1], d[2], d[3]);
+                else
+                {
+                    sR[q] = make_double2(d[0], d[1]);
+                    sR[T::RPL + q] = make_double2(d[2], d[3]);
+                }
+            };
+            if (inM) jump(rM, sideM, true, FL);
+            if (inP) jump(rP, sideP, false, FR);
+        }
+    }
+    __syncthreads();
+
+    // ---- row pass: one row of element e, in place
+    if (own)
+    {
+        const int mr = T::ROT ? (m + T::ROT * e) % N : m;
+        const int at = e * T::ES + mr * T::RS;
+        S dl[4], dr[4];
+        get_jump(e * T::DS + mr, dl);
+        get_jump(e * T::DS + T::oR + mr, dr);
+#pragma unroll
+        for (int pl = 0; pl < T::NP; ++pl)
+        {
+            constexpr int W = F32 ? 4 : 2;
+            V* f = sF + pl * T::PLANE + at;
+            S x[W][N], y[AFF ? 1 : W][N];
+#pragma unroll
+            for (int q = 0; q < N; ++q)
+            {
+                const V t = f[q];
+                x[0][q] = t.x; x[1][q] = t.y;
+                if constexpr (F32) { x[2][q] = t.z; x[3][q] = t.w; }
+                if constexpr (!AFF)
+                {
+                    const V u = sG[pl * T::PLANE + at + q];
+                    y[0][q] = u.x; y[1][q] = u.y;
+                    if constexpr (F32) { y[2][q] = u.z; y[3][q] = u.w; }
+                }
+            }
+#pragma unroll
+            for (int w = 0; w < W; ++w)
+            {
+                center_line<S, N>(x[w]);
+                if constexpr (!AFF) center_line<S, N>(y[w]);
+            }
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+            {
+                S r[W];
+                double2 mx = make_double2(0.0, 0.0);
+                if constexpr (!AFF) mx = __ldg(reinterpret_cast<const double2*>(a.metrics + (mbase + mr * N + k) * 4));
+#pragma unroll
+                for (int w = 0; w < W; ++w)
+                {
+                    const int eq = W * pl + w;
+                    S d = S(0.0);
+#pragma unroll
+                    for (int q = 0; q < N; ++q) d = d + opD<S>(ops, k * N + q) * x[w][q];
+                    if constexpr (!AFF)
+                    {
+                        S h = S(0.0);
+#pragma unroll
+                        for (int q = 0; q < N; ++q) h = h + opD<S>(ops, k * N + q) * y[w][q];
+                        r[w] = ((S(mx.x) * d + S(mx.y) * h) + dl[eq] * opL<S>(ops, k)) + dr[eq] * opR<S>(ops, k);
+                    }
+                    else  // xi_x is also the scale of the jumps
+                        r[w] = S(a.xi_x) * ((d + dl[eq] * opL<S>(ops, k)) + dr[eq] * opR<S>(ops, k));
+                }
+                if constexpr (F32) f[k] = make_float4(r[0], r[1], r[2], r[3]);
+                else f[k] = make_double2(r[0], r[1]);
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- output pass: column m of element e
+    if (own)
+    {
+        S b[4], t[4];
+        get_jump(e * T::DS + T::oB + m, b);
+        get_jump(e * T::DS + T::oT + m, t);
+        if constexpr (AFF)
+        {
+            // from the y-faces' frame: (d0, dn, dt, d3) to (d0, -dt, dn, d3)
+            const S bn = b[1], tn = t[1];
+            b[1] = -b[2];
+            b[2] = bn;
+            t[1] = -t[2];
+            t[2] = tn;
+        }
+#pragma unroll
+        for (int l = 0; l < N; ++l)
+        {
+            S x[4];
+            get_flux(sF, e * T::ES + l * T::RS + m, x);
+            const S dLl = opL<S>(ops, l), dRl = opR<S>(ops, l);
+#pragma unroll
+            for (int eq = 0; eq < 4; ++eq)
+                // affine: eta_y is also the scale of the jumps
+                E[eq][l] = AFF ? x[eq] + S(a.eta_y) * ((E[eq][l] + b[eq] * dLl) + t[eq] * dRl)
+                               : ((x[eq] + E[eq][l]) + b[eq] * dLl) + t[eq] * dRl;
+        }
+    }
+    if constexpr (F32)
+    {
+        if (own)
+        {
+            float4* o = reinterpret_cast<float4*>(static_cast<float*>(a.out) + ebase + m * 4);
+#pragma unroll
+            for (int l = 0; l < N; ++l) o[l * N] = make_float4(E[0][l], E[1][l], E[2][l], E[3][l]);
+        }
+    }
+    else
+        line_output<T, N, GAS, POST>(a, ops, own, e, m, ebase, i0, j0, txe, tye, E, sF);
+}
+
+template <class S, int N, int GAS, int RIEM, int GEO, int VAR, bool POST>
+__global__ void __launch_bounds__((Line2D<N, GEO, VAR, S>::BT), (Line2D<N, GEO, VAR, S>::CTAS))
     fr2d_line_kernel(const __grid_constant__ Fr2dArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -833,18 +936,18 @@ __global__ void __launch_bounds__((Line2D<N, GEO, VAR>::BT), (Line2D<N, GEO, VAR
     {
         // the state of the tile one residency ahead into L2 (hints): its CTA starts on this
         // one's shared memory and registers, and finds its loads near
-        using T = Line2D<N, GEO, VAR>;
+        using T = Line2D<N, GEO, VAR, S>;
         const int nb = int(blockIdx.y * gridDim.x + blockIdx.x) + T::CTAS * kSMs;
         const int by = nb / int(gridDim.x), bx = nb - by * int(gridDim.x);
-        constexpr int LROW = (T::TX * T::ND * int(sizeof(double)) + 127) / 128;
+        constexpr int LROW = (T::TX * T::ND * int(sizeof(S)) + 127) / 128, LV = 128 / int(sizeof(S));
         for (int q = threadIdx.x; q < T::TY * LROW; q += T::BT)
         {
             const int y = q / LROW, ln = q % LROW, j = by * T::TY + a.row_begin + y;
-            if (j < a.row_end && bx * T::TX * T::ND + ln * 16 < a.Nx * T::ND)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(a.U + (int64_t(j) * a.Nx + bx * T::TX) * T::ND + ln * 16));
+            if (j < a.row_end && bx * T::TX * T::ND + ln * LV < a.Nx * T::ND)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const S*>(a.U) + (int64_t(j) * a.Nx + bx * T::TX) * T::ND + ln * LV));
         }
     }
-    fr2d_line_tile<N, GAS, RIEM, GEO, VAR, POST>(a, a.ops, blockIdx.x, blockIdx.y, smem_raw);
+    fr2d_line_tile<S, N, GAS, RIEM, GEO, VAR, POST>(a, a.ops, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 // Kernel attributes are per device: set once on each device that launches.
@@ -862,10 +965,11 @@ template <class K> cudaError_t set_smem_once(K kern, size_t bytes, bool (&done)[
     return cudaSuccess;
 }
 
-template <int N, int GAS, int RIEM, int GEO, int VAR, bool POST> cudaError_t launch_line_v(const Fr2dArgs& a, cudaStream_t st)
+template <class S, int N, int GAS, int RIEM, int GEO, int VAR, bool POST>
+cudaError_t launch_line_v(const Fr2dArgs& a, cudaStream_t st)
 {
-    using T = Line2D<N, GEO, VAR>;
-    auto kern = fr2d_line_kernel<N, GAS, RIEM, GEO, VAR, POST>;
+    using T = Line2D<N, GEO, VAR, S>;
+    auto kern = fr2d_line_kernel<S, N, GAS, RIEM, GEO, VAR, POST>;
     static bool done[64] = {};
     const cudaError_t e = set_smem_once(kern, T::bytes, done);
     if (e != cudaSuccess) return e;
@@ -880,14 +984,17 @@ template <int N, int GAS, int RIEM, int GEO, int VAR, bool POST> cudaError_t lau
 // residency the tuned tile does less halo work per element (96^2: p = 3 8.1 -> 7.4, p = 5
 // 12.9 -> 10.5 us).  Curved p = 5, whose tuned tile fills few warps, takes it at any size (256^2
 // vortex 0.143 -> 0.126 ms).
-template <int N, int GAS, int RIEM, int GEO> cudaError_t launch_line(const Fr2dArgs& a, cudaStream_t st)
+template <class S, int N, int GAS, int RIEM, int GEO> cudaError_t launch_line(const Fr2dArgs& a, cudaStream_t st)
 {
-    const bool post = a.mode == MODE_STAGE && a.post;
-    using S = Line2D<N, GEO, 2>;
-    const int64_t tiles = int64_t((a.Nx + S::TX - 1) / S::TX) * ((a.row_end - a.row_begin + S::TY - 1) / S::TY);
-    if (tiles <= S::CTAS * kSMs || (GEO == GEO_CURVED && N == 6))
-        return post ? launch_line_v<N, GAS, RIEM, GEO, 2, true>(a, st) : launch_line_v<N, GAS, RIEM, GEO, 2, false>(a, st);
-    return post ? launch_line_v<N, GAS, RIEM, GEO, 0, true>(a, st) : launch_line_v<N, GAS, RIEM, GEO, 0, false>(a, st);
+    using L = Line2D<N, GEO, 2, S>;
+    const int64_t tiles = int64_t((a.Nx + L::TX - 1) / L::TX) * ((a.row_end - a.row_begin + L::TY - 1) / L::TY);
+    const bool small = tiles <= L::CTAS * kSMs || (GEO == GEO_CURVED && N == 6 && !L::F32);
+    if constexpr (!L::F32)
+    {
+        if (a.mode == MODE_STAGE && a.post)
+            return small ? launch_line_v<S, N, GAS, RIEM, GEO, 2, true>(a, st) : launch_line_v<S, N, GAS, RIEM, GEO, 0, true>(a, st);
+    }
+    return small ? launch_line_v<S, N, GAS, RIEM, GEO, 2, false>(a, st) : launch_line_v<S, N, GAS, RIEM, GEO, 0, false>(a, st);
 }
 
 } // namespace frsdg

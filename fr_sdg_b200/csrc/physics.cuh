@@ -333,56 +333,56 @@ __device__ __forceinline__ void riemann_rec(const S L[RF_N], const S R[RF_N], do
 // (riemann_solver.hpp:314-341) as one choice of side K and one of star state or F_K: the
 // outer states are F_L when s_L >= 0 and F_R when neither s_M nor s_R is non-negative, and
 // K is that side in both.
-template <int RIEM, int AXIS, class M>
-__device__ __forceinline__ void riemann_sides(const double L[RF_N], const double R[RF_N], double nx, double ny,
-                                              double Fs[4], double FnL[4], double FnR[4], const M& m)
+template <int RIEM, int AXIS, class S, class M>
+__device__ __forceinline__ void riemann_sides(const S L[RF_N], const S R[RF_N], S nx, S ny, S Fs[4], S FnL[4],
+                                              S FnR[4], const M& m)
 {
-    const double unL = AXIS == 0 ? L[RF_U] : AXIS == 1 ? L[RF_V] : L[RF_U] * nx + L[RF_V] * ny;
-    const double utL = AXIS == 0 ? L[RF_V] : AXIS == 1 ? -L[RF_U] : -L[RF_U] * ny + L[RF_V] * nx;
-    const double unR = AXIS == 0 ? R[RF_U] : AXIS == 1 ? R[RF_V] : R[RF_U] * nx + R[RF_V] * ny;
-    const double utR = AXIS == 0 ? R[RF_V] : AXIS == 1 ? -R[RF_U] : -R[RF_U] * ny + R[RF_V] * nx;
-    const double cL = L[RF_C], cR = R[RF_C], pL = L[RF_P], pR = R[RF_P];
+    const S unL = AXIS == 0 ? L[RF_U] : AXIS == 1 ? L[RF_V] : L[RF_U] * nx + L[RF_V] * ny;
+    const S utL = AXIS == 0 ? L[RF_V] : AXIS == 1 ? -L[RF_U] : -L[RF_U] * ny + L[RF_V] * nx;
+    const S unR = AXIS == 0 ? R[RF_U] : AXIS == 1 ? R[RF_V] : R[RF_U] * nx + R[RF_V] * ny;
+    const S utR = AXIS == 0 ? R[RF_V] : AXIS == 1 ? -R[RF_U] : -R[RF_U] * ny + R[RF_V] * nx;
+    const S cL = L[RF_C], cR = R[RF_C], pL = L[RF_P], pR = R[RF_P];
     // fluxes in the frame (n, t)
-    const double FL0 = L[RF_RHO] * unL, FR0 = R[RF_RHO] * unR;
-    const double FL[4] = {FL0, FL0 * unL + pL, FL0 * utL, (L[RF_E] + pL) * unL};
-    const double FR[4] = {FR0, FR0 * unR + pR, FR0 * utR, (R[RF_E] + pR) * unR};
-    double f[4];
+    const S FL0 = L[RF_RHO] * unL, FR0 = R[RF_RHO] * unR;
+    const S FL[4] = {FL0, FL0 * unL + pL, FL0 * utL, (L[RF_E] + pL) * unL};
+    const S FR[4] = {FR0, FR0 * unR + pR, FR0 * utR, (R[RF_E] + pR) * unR};
+    S f[4];
     if constexpr (RIEM == FRSDG_RUSANOV)
     {
-        const double hs = 0.5 * smooth_max(smooth_abs(unL, m) + cL, smooth_abs(unR, m) + cR, m);
-        f[0] = 0.5 * (FL[0] + FR[0]) - hs * (R[RF_RHO] - L[RF_RHO]);
-        f[1] = 0.5 * (FL[1] + FR[1]) - hs * (FR0 - FL0);
-        f[2] = 0.5 * (FL[2] + FR[2]) - hs * (R[RF_RHO] * utR - L[RF_RHO] * utL);
-        f[3] = 0.5 * (FL[3] + FR[3]) - hs * (R[RF_E] - L[RF_E]);
+        const S hs = cs<S>(0.5) * smooth_max(smooth_abs(unL, m) + cL, smooth_abs(unR, m) + cR, m);
+        f[0] = cs<S>(0.5) * (FL[0] + FR[0]) - hs * (R[RF_RHO] - L[RF_RHO]);
+        f[1] = cs<S>(0.5) * (FL[1] + FR[1]) - hs * (FR0 - FL0);
+        f[2] = cs<S>(0.5) * (FL[2] + FR[2]) - hs * (R[RF_RHO] * utR - L[RF_RHO] * utL);
+        f[3] = cs<S>(0.5) * (FL[3] + FR[3]) - hs * (R[RF_E] - L[RF_E]);
     }
     else
     {
-        const double sL = smooth_min(unL - cL, unR - cR, m);
-        const double sR = smooth_max(unL + cL, unR + cR, m);
-        const double dL = L[RF_RHO] * (sL - unL);
-        const double dR = R[RF_RHO] * (sR - unR);
-        const double sM = (pR - pL + unL * dL - unR * dR) * m.rcp(dL - dR);
-        const bool takeL = sL >= 0.0, left = sM >= 0.0;
+        const S sL = smooth_min(unL - cL, unR - cR, m);
+        const S sR = smooth_max(unL + cL, unR + cR, m);
+        const S dL = L[RF_RHO] * (sL - unL);
+        const S dR = R[RF_RHO] * (sR - unR);
+        const S sM = (pR - pL + unL * dL - unR * dR) * m.rcp(dL - dR);
+        const bool takeL = sL >= cs<S>(0.0), left = sM >= cs<S>(0.0);
         const bool k = takeL || left;                         // K = L
-        const bool outer = takeL || !(left || sR >= 0.0);     // F_K itself
-        const double K0 = k ? L[RF_RHO] : R[RF_RHO];
-        const double K3 = k ? L[RF_E] : R[RF_E];
-        const double sK = k ? sL : sR;
-        const double unK = k ? unL : unR;
-        const double utK = k ? utL : utR;
-        const double pK = k ? pL : pR;
-        const double FK0 = K0 * unK, FK1 = FK0 * unK + pK, FK3 = (K3 + pK) * unK;
-        const double ps = sK * (pK + K0 * (sK - unK) * (sM - unK));
-        const double inv = m.rcp(sK - sM);
-        const double st0 = (sM * (sK * K0 - FK0)) * inv;
-        const double st1 = (sM * (sK * FK0 - FK1) + ps) * inv;
-        const double st3 = (sM * (sK * K3 - FK3) + ps * sM) * inv;
+        const bool outer = takeL || !(left || sR >= cs<S>(0.0));     // F_K itself
+        const S K0 = k ? L[RF_RHO] : R[RF_RHO];
+        const S K3 = k ? L[RF_E] : R[RF_E];
+        const S sK = k ? sL : sR;
+        const S unK = k ? unL : unR;
+        const S utK = k ? utL : utR;
+        const S pK = k ? pL : pR;
+        const S FK0 = K0 * unK, FK1 = FK0 * unK + pK, FK3 = (K3 + pK) * unK;
+        const S ps = sK * (pK + K0 * (sK - unK) * (sM - unK));
+        const S inv = m.rcp(sK - sM);
+        const S st0 = (sM * (sK * K0 - FK0)) * inv;
+        const S st1 = (sM * (sK * FK0 - FK1) + ps) * inv;
+        const S st3 = (sM * (sK * K3 - FK3) + ps * sM) * inv;
         f[0] = outer ? FK0 : st0;
         f[1] = outer ? FK1 : st1;
         f[2] = utK * f[0];
         f[3] = outer ? FK3 : st3;
     }
-    auto back = [&](const double v[4], double o[4]) {
+    auto back = [&](const S v[4], S o[4]) {
         o[0] = v[0];
         o[1] = AXIS == 0 ? v[1] : AXIS == 1 ? -v[2] : v[1] * nx - v[2] * ny;
         o[2] = AXIS == 0 ? v[2] : AXIS == 1 ? v[1] : v[1] * ny + v[2] * nx;

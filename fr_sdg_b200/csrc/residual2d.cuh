@@ -393,6 +393,21 @@ __device__ __forceinline__ void face_ghost(const Fr2dArgs& a, int i0, int j0, Fa
     }
 }
 
+// FP32 derivatives: the rows of the rounded differentiation matrix do not sum to zero
+// exactly, so a line's constant part (a uniform background flux) would leave a residual
+// of ~1e-7 |F| |D| at every node, the same sign every step.  Differentiating the line
+// minus its first value removes that bias (D 1 = 0 in exact arithmetic, so the result
+// is unchanged otherwise).  FP64 keeps the reference's form.
+template <class S, int N> __device__ __forceinline__ void center_line(S (&v)[N])
+{
+    if constexpr (sizeof(S) == 4)
+    {
+        const S b = v[0];
+#pragma unroll
+        for (int m = 0; m < N; ++m) v[m] = v[m] - b;
+    }
+}
+
 } // namespace frsdg
 #include "line2d.cuh"
 namespace frsdg
@@ -552,21 +567,6 @@ __device__ __forceinline__ void stage_epilogue(const Fr2dArgs& a, const Ops& ops
 
 // One tile of the residual pass: tile (bx, by) of element columns/rows, with the launch arguments `a` and the operators
 // `ops`; smem_raw is the CTA's dynamic shared memory (T::bytes).
-// FP32 derivatives: the rows of the rounded differentiation matrix do not sum to zero
-// exactly, so a line's constant part (a uniform background flux) would leave a residual
-// of ~1e-7 |F| |D| at every node, the same sign every step.  Differentiating the line
-// minus its first value removes that bias (D 1 = 0 in exact arithmetic, so the result
-// is unchanged otherwise).  FP64 keeps the reference's form.
-template <class S, int N> __device__ __forceinline__ void center_line(S (&v)[N])
-{
-    if constexpr (sizeof(S) == 4)
-    {
-        const S b = v[0];
-#pragma unroll
-        for (int m = 0; m < N; ++m) v[m] = v[m] - b;
-    }
-}
-
 // POST: the instantiation with the stage epilogue (Fr2dArgs::post); the others carry no
 // epilogue code, which would otherwise cost the main path registers.
 template <class S, int N, int GAS, int RIEM, int GEO, int VAR, bool POST = false, bool TC = false>
@@ -1182,8 +1182,17 @@ cudaError_t launch_fr2d_tiles(const Fr2dArgs& a, cudaStream_t st)
 template <class S, int N, int GAS, int RIEM, int GEO>
 cudaError_t launch_fr2d_kernel(const Fr2dArgs& a, cudaStream_t st)
 {
-    if constexpr (std::is_same<S, double>::value) return launch_line<N, GAS, RIEM, GEO>(a, st);
-    else return launch_fr2d_tiles<S, N, GAS, RIEM, GEO>(a, st);
+    if constexpr (std::is_same<S, double>::value) return launch_line<S, N, GAS, RIEM, GEO>(a, st);
+    else
+    {
+        if constexpr (std::is_same<S, float>::value)
+        {
+            // an FP32 state's residual; the mixed stages (FP64 input, primitives recovered in
+            // FP64) and the tensor-core contractions keep the tiles
+            if (!a.in_f64 && !a.tc && a.mode == MODE_RESIDUAL && a.out_f32) return launch_line<S, N, GAS, RIEM, GEO>(a, st);
+        }
+        return launch_fr2d_tiles<S, N, GAS, RIEM, GEO>(a, st);
+    }
 }
 
 // ---- batches ------------------------------------------------------------------
@@ -1291,7 +1300,7 @@ __global__ void __launch_bounds__((Line2D<N, GEO_AFFINE, VAR>::BT), (Line2D<N, G
         __syncthreads();
         if (threadIdx.x == 0) batch_stage_args(sa, in, ck, b.stage, b.mixed != 0);
         __syncthreads();
-        fr2d_line_tile<N, GAS, RIEM, GEO_AFFINE, VAR, POST>(sa, b.ops, tm.y, tm.z, smem_raw);
+        fr2d_line_tile<double, N, GAS, RIEM, GEO_AFFINE, VAR, POST>(sa, b.ops, tm.y, tm.z, smem_raw);
     }
 }
 
