@@ -13,6 +13,9 @@
 //                      least-squares problem turns with it; 1/hn (0 at breakdown) scales
 //                      the next basis vector;
 //   back substitution  y = R^-1 g at the end of a cycle (R the rotated Hessenberg).
+// One step is six launches and reads the basis three times: the update of the first pass
+// takes the second pass's dot products along (1,048,576 unknowns, j = 5, 15, 30: 60, 171, 308 -> 33, 109,
+// 209 us against eleven launches and four reads).
 // Reductions are two-stage (per-block partial sums in a fixed order, then one block per
 // sum), so repeated solves give identical bits.  Every kernel reads its sizes from the
 // arguments; scratch is the caller's `work` array (frsdg_gmres_work_doubles).
@@ -34,8 +37,7 @@ constexpr int kKryMaxBasis = 256;                           // Arnoldi vectors p
 static int64_t kry_blocks(int64_t n) { return (n + kKryChunk - 1) / kKryChunk; }
 
 // work layout (doubles): part[(kKryMaxBasis + 1) * B] | h1[kKryMaxBasis] | h2[kKryMaxBasis] |
-// scalars[4] (0: ||w||^2 before, 1: ||w||^2 after the first pass, 2: reorthogonalise
-// flag as 0/1, 3: ||w||^2 after the second pass)
+// scalars[4] (0: ||w||^2 before, 1: ||w||^2 after the first pass; 2, 3 unused)
 struct KryWork
 {
     double* part;
@@ -68,122 +70,210 @@ __device__ __forceinline__ double block_sum(double v, double* red)
     return s;  // valid on thread 0
 }
 
-// Per-block partial dot products of w with V[0..nv) (and w.w when with_norm) into
-// part[i * B + block]; skipped unless the flag (when given) is set.
-__global__ void __launch_bounds__(kKryThreads) kry_dot_kernel(const double* V, int64_t ldv, int nv, const double* w,
-                                                               int64_t n, double* part, int with_norm,
-                                                               const double* flag)
+__device__ __forceinline__ double warp_sum(double v)
 {
-    if (flag && *flag == 0.0) return;
-    __shared__ double red[kKryThreads / 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;  // valid on lane 0
+}
+
+constexpr int kKryWarps = kKryThreads / 32;
+
+// The block's sums red[i * warps + warp], i in [0, nv), to part[i * B + block].
+__device__ __forceinline__ void store_partials(const double* red, int nv, double* part)
+{
+    __syncthreads();
+    for (int i = threadIdx.x; i < nv; i += kKryThreads)
+    {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < kKryWarps; ++q) s += red[i * kKryWarps + q];
+        part[int64_t(i) * gridDim.x + blockIdx.x] = s;
+    }
+}
+
+// Per-block partial dot products of w with V[0..nv) and of w with itself, into
+// part[i * B + block] (w at i = nv).  Each warp leaves its sums in its own slots, so the
+// block meets once.
+__global__ void __launch_bounds__(kKryThreads) kry_dot_kernel(const double* V, int64_t ldv, int nv, const double* w,
+                                                               int64_t n, double* part)
+{
+    __shared__ double red[(kKryMaxBasis + 1) * kKryWarps];
     const int64_t base = int64_t(blockIdx.x) * kKryChunk + threadIdx.x;
-    const int64_t B = gridDim.x;
-    double wv[kKryPerThread];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double wv[kKryPerThread], s = 0.0;
 #pragma unroll
     for (int k = 0; k < kKryPerThread; ++k)
     {
         const int64_t e = base + int64_t(k) * kKryThreads;
         wv[k] = e < n ? w[e] : 0.0;
+        s = fma(wv[k], wv[k], s);
     }
-    if (with_norm)
-    {
-        double s = 0.0;
-#pragma unroll
-        for (int k = 0; k < kKryPerThread; ++k) s = fma(wv[k], wv[k], s);
-        s = block_sum(s, red);
-        if (threadIdx.x == 0) part[int64_t(nv) * B + blockIdx.x] = s;
-    }
+    s = warp_sum(s);
+    if (lane == 0) red[nv * kKryWarps + warp] = s;
+#pragma unroll 2
     for (int i = 0; i < nv; ++i)
     {
         const double* v = V + int64_t(i) * ldv;
-        double s = 0.0;
+        double d = 0.0;
 #pragma unroll
         for (int k = 0; k < kKryPerThread; ++k)
         {
             const int64_t e = base + int64_t(k) * kKryThreads;
-            if (e < n) s = fma(__ldg(v + e), wv[k], s);
+            if (e < n) d = fma(__ldg(v + e), wv[k], d);
         }
-        s = block_sum(s, red);
-        if (threadIdx.x == 0) part[int64_t(i) * B + blockIdx.x] = s;
+        d = warp_sum(d);
+        if (lane == 0) red[i * kKryWarps + warp] = d;
     }
+    store_partials(red, nv + 1, part);
 }
 
-// w <- w - sum_i h[i] V[i]; per-block partial ||w||^2 into part[nv * B + block].
+// w <- w - sum_i h[i] V[i], then the next pass's partial dot products of the new w with V and
+// its partial ||w||^2 (row nv of part): the block works through its chunk in pieces of 512
+// entries, whose columns of V the dot products find in cache, so the two passes read V from
+// memory once.
+__global__ void __launch_bounds__(kKryThreads) kry_update_dot_kernel(const double* V, int64_t ldv, int nv, double* w,
+                                                                      int64_t n, const double* h, double* part)
+{
+    __shared__ double red[(kKryMaxBasis + 1) * kKryWarps];
+    __shared__ double sh[kKryMaxBasis];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < nv; i += kKryThreads) sh[i] = h[i];
+    for (int i = lane; i < nv; i += 32) red[i * kKryWarps + warp] = 0.0;
+    __syncthreads();
+    double s = 0.0;
+#pragma unroll 1
+    for (int q = 0; q < kKryPerThread; q += 2)
+    {
+        const int64_t e0 = int64_t(blockIdx.x) * kKryChunk + q * kKryThreads + threadIdx.x, e1 = e0 + kKryThreads;
+        const bool in0 = e0 < n, in1 = e1 < n;
+        double a0 = in0 ? w[e0] : 0.0, a1 = in1 ? w[e1] : 0.0;
+#pragma unroll 4
+        for (int i = 0; i < nv; ++i)
+        {
+            const double* v = V + int64_t(i) * ldv;
+            a0 = fma(-sh[i], in0 ? __ldg(v + e0) : 0.0, a0);
+            a1 = fma(-sh[i], in1 ? __ldg(v + e1) : 0.0, a1);
+        }
+        if (in0) w[e0] = a0;
+        if (in1) w[e1] = a1;
+        s = fma(a0, a0, fma(a1, a1, s));
+#pragma unroll 4
+        for (int i = 0; i < nv; ++i)
+        {
+            const double* v = V + int64_t(i) * ldv;
+            double d = in0 ? __ldg(v + e0) * a0 : 0.0;
+            if (in1) d = fma(__ldg(v + e1), a1, d);
+            d = warp_sum(d);
+            if (lane == 0) red[i * kKryWarps + warp] += d;
+        }
+    }
+    s = warp_sum(s);
+    if (lane == 0) red[nv * kKryWarps + warp] = s;
+    store_partials(red, nv + 1, part);
+}
+
+// Whether the second pass acts: ||w||^2 fell below half its value in the first.
+__device__ __forceinline__ bool kry_again(const double* sc) { return sc[1] < 0.5 * sc[0]; }
+
+// The second pass: w <- w - sum_i h[i] V[i] and the partial ||w||^2 into row nv of part.
 __global__ void __launch_bounds__(kKryThreads) kry_update_kernel(const double* V, int64_t ldv, int nv, double* w,
                                                                   int64_t n, const double* h, double* part,
-                                                                  const double* flag)
+                                                                  const double* sc)
 {
-    if (flag && *flag == 0.0) return;
-    __shared__ double red[kKryThreads / 32];
+    if (!kry_again(sc)) return;
+    __shared__ double red[kKryWarps];
     __shared__ double sh[kKryMaxBasis];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < nv; i += kKryThreads) sh[i] = h[i];
     __syncthreads();
-    const int64_t base = int64_t(blockIdx.x) * kKryChunk + threadIdx.x;
-    const int64_t B = gridDim.x;
     double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < kKryPerThread; ++k)
+#pragma unroll 1
+    for (int q = 0; q < kKryPerThread; q += 4)
     {
-        const int64_t e = base + int64_t(k) * kKryThreads;
-        if (e < n)
+        const int64_t e0 = int64_t(blockIdx.x) * kKryChunk + q * kKryThreads + threadIdx.x;
+        double a[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[k] = e0 + k * kKryThreads < n ? w[e0 + k * kKryThreads] : 0.0;
+#pragma unroll 2
+        for (int i = 0; i < nv; ++i)
         {
-            double acc = w[e];
-            for (int i = 0; i < nv; ++i) acc = fma(-sh[i], __ldg(V + int64_t(i) * ldv + e), acc);
-            w[e] = acc;
-            s = fma(acc, acc, s);
+            const double* v = V + int64_t(i) * ldv + e0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (e0 + k * kKryThreads < n) a[k] = fma(-sh[i], __ldg(v + k * kKryThreads), a[k]);
         }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (e0 + k * kKryThreads < n)
+            {
+                w[e0 + k * kKryThreads] = a[k];
+                s = fma(a[k], a[k], s);
+            }
     }
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) part[int64_t(nv) * B + blockIdx.x] = s;
+    s = warp_sum(s);
+    if (lane == 0) red[warp] = s;
+    store_partials(red, 1, part + int64_t(nv) * gridDim.x);
 }
 
-// One block per sum: out[i] = sum_b part[i * B + b] for i in [0, count), in a fixed order.
-__global__ void __launch_bounds__(kKryThreads) kry_reduce_kernel(const double* part, int64_t B, double* out,
-                                                                  const double* flag)
+// One block per sum: the sum of part[i * B ...] over its B entries to out[i] for i < nv and to
+// *last for i = nv, in a fixed order.
+__global__ void __launch_bounds__(kKryThreads) kry_reduce_kernel(const double* part, int64_t B, int nv, double* out,
+                                                                  double* last)
 {
-    if (flag && *flag == 0.0) return;
     __shared__ double red[kKryThreads / 32];
     const double* p = part + int64_t(blockIdx.x) * B;
     double s = 0.0;
     for (int64_t b = threadIdx.x; b < B; b += kKryThreads) s += p[b];
     s = block_sum(s, red);
-    if (threadIdx.x == 0) out[blockIdx.x] = s;
-}
-
-// After the first pass: reorthogonalise when ||w||^2 fell below half its value.
-__global__ void kry_dgks_kernel(double* sc)
-{
-    sc[2] = sc[1] < 0.5 * sc[0] ? 1.0 : 0.0;
+    if (threadIdx.x == 0) (int(blockIdx.x) < nv ? out + blockIdx.x : last)[0] = s;
 }
 
 // The new Hessenberg column j: H[0..j][j] = h1 + h2 (h2 only after a second pass),
-// H[j+1][j] = ||w||; the previous rotations, the new one, the residual vector g, and
-// 1/||w|| (0 when w vanished) for the next basis vector.  H is row-major with leading
-// dimension ldh.
-__global__ void kry_givens_kernel(double* H, int ldh, double* cs, double* sn, double* g, const double* h1,
-                                  const double* h2, const double* sc, int j, double* inv_hn)
+// H[j+1][j] = ||w|| (after a second pass from its B partial sums `norm`); the previous
+// rotations, the new one, the residual vector g, and 1/||w|| (0 when w vanished) for the next
+// basis vector.  H is row-major with leading dimension ldh.  One block: the sum and the
+// column's entries in parallel, the rotations on one thread from shared memory.
+__global__ void __launch_bounds__(kKryThreads) kry_givens_kernel(double* H, int ldh, double* cs, double* sn, double* g,
+                                                                  const double* h1, const double* h2, const double* sc,
+                                                                  const double* norm, int64_t B, int j, double* inv_hn)
 {
-    const bool second = sc[2] != 0.0;
-    for (int i = 0; i <= j; ++i) H[int64_t(i) * ldh + j] = second ? h1[i] + h2[i] : h1[i];
-    const double nrm2 = second ? sc[3] : sc[1];
-    const double hn = sqrt(nrm2 > 0.0 ? nrm2 : 0.0);
-    H[int64_t(j + 1) * ldh + j] = hn;
-    for (int i = 0; i < j; ++i)
+    __shared__ double red[kKryThreads / 32];
+    __shared__ double col[kKryMaxBasis + 1], c_[kKryMaxBasis], s_[kKryMaxBasis];
+    const bool second = kry_again(sc);
+    for (int i = threadIdx.x; i <= j; i += kKryThreads) col[i] = second ? h1[i] + h2[i] : h1[i];
+    for (int i = threadIdx.x; i < j; i += kKryThreads)
     {
-        const double a = H[int64_t(i) * ldh + j], b = H[int64_t(i + 1) * ldh + j];
-        H[int64_t(i) * ldh + j] = cs[i] * a + sn[i] * b;
-        H[int64_t(i + 1) * ldh + j] = -sn[i] * a + cs[i] * b;
+        c_[i] = cs[i];
+        s_[i] = sn[i];
     }
-    const double a = H[int64_t(j) * ldh + j], b = H[int64_t(j + 1) * ldh + j];
-    const double den = hypot(a, b);
-    const double c = den == 0.0 ? 1.0 : a / den, s = den == 0.0 ? 0.0 : b / den;
-    cs[j] = c;
-    sn[j] = s;
-    H[int64_t(j) * ldh + j] = c * a + s * b;
-    H[int64_t(j + 1) * ldh + j] = 0.0;
-    g[j + 1] = -s * g[j];
-    g[j] = c * g[j];
-    *inv_hn = hn > 0.0 ? 1.0 / hn : 0.0;
+    double v = 0.0;
+    if (second)
+        for (int64_t b = threadIdx.x; b < B; b += kKryThreads) v += norm[b];
+    v = block_sum(v, red);  // its barriers also order the shared column
+    if (threadIdx.x == 0)
+    {
+        const double nrm2 = second ? v : sc[1];
+        const double hn = sqrt(nrm2 > 0.0 ? nrm2 : 0.0);
+        double a = col[0];
+        for (int i = 0; i < j; ++i)
+        {
+            const double b = col[i + 1];
+            col[i] = c_[i] * a + s_[i] * b;
+            a = -s_[i] * a + c_[i] * b;
+        }
+        const double b = hn;
+        const double den = hypot(a, b);
+        const double c = den == 0.0 ? 1.0 : a / den, s = den == 0.0 ? 0.0 : b / den;
+        cs[j] = c;
+        sn[j] = s;
+        col[j] = c * a + s * b;
+        g[j + 1] = -s * g[j];
+        g[j] = c * g[j];
+        *inv_hn = hn > 0.0 ? 1.0 / hn : 0.0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i <= j + 1; i += kKryThreads) H[int64_t(i) * ldh + j] = i <= j ? col[i] : 0.0;
 }
 
 // y = R^-1 g over the first k columns; a zero diagonal (columns after a breakdown)
@@ -222,19 +312,15 @@ int frsdg_gmres_arnoldi(const double* V, int64_t ldv, int32_t j, double* w, int6
     const KryWork k = kry_work(work, B);
     const int nv = j + 1;
     const unsigned grid = unsigned(B);
-    // first pass: h1 = V^T w and ||w||^2 (sc[0]); w -= V h1 and ||w||^2 (sc[1])
-    kry_dot_kernel<<<grid, kKryThreads, 0, s>>>(V, ldv, nv, w, n, k.part, 1, nullptr);
-    kry_reduce_kernel<<<unsigned(nv), kKryThreads, 0, s>>>(k.part, B, k.h1, nullptr);
-    kry_reduce_kernel<<<1, kKryThreads, 0, s>>>(k.part + int64_t(nv) * B, B, k.sc, nullptr);
-    kry_update_kernel<<<grid, kKryThreads, 0, s>>>(V, ldv, nv, w, n, k.h1, k.part, nullptr);
-    kry_reduce_kernel<<<1, kKryThreads, 0, s>>>(k.part + int64_t(nv) * B, B, k.sc + 1, nullptr);
-    kry_dgks_kernel<<<1, 1, 0, s>>>(k.sc);
-    // second pass when flagged: h2, w -= V h2, ||w||^2 (sc[3])
-    kry_dot_kernel<<<grid, kKryThreads, 0, s>>>(V, ldv, nv, w, n, k.part, 0, k.sc + 2);
-    kry_reduce_kernel<<<unsigned(nv), kKryThreads, 0, s>>>(k.part, B, k.h2, k.sc + 2);
-    kry_update_kernel<<<grid, kKryThreads, 0, s>>>(V, ldv, nv, w, n, k.h2, k.part, k.sc + 2);
-    kry_reduce_kernel<<<1, kKryThreads, 0, s>>>(k.part + int64_t(nv) * B, B, k.sc + 3, k.sc + 2);
-    kry_givens_kernel<<<1, 1, 0, s>>>(H, ldh, cs, sn, g, k.h1, k.h2, k.sc, j, inv_hn);
+    const double* norm = k.part + int64_t(nv) * B;
+    // first pass: h1 = V^T w and ||w||^2 (sc[0]); w -= V h1, its ||w||^2 (sc[1]) and h2 = V^T w
+    kry_dot_kernel<<<grid, kKryThreads, 0, s>>>(V, ldv, nv, w, n, k.part);
+    kry_reduce_kernel<<<unsigned(nv) + 1, kKryThreads, 0, s>>>(k.part, B, nv, k.h1, k.sc);
+    kry_update_dot_kernel<<<grid, kKryThreads, 0, s>>>(V, ldv, nv, w, n, k.h1, k.part);
+    kry_reduce_kernel<<<unsigned(nv) + 1, kKryThreads, 0, s>>>(k.part, B, nv, k.h2, k.sc + 1);
+    // second pass when the first shrank w (kry_again): w -= V h2 and its ||w||^2
+    kry_update_kernel<<<grid, kKryThreads, 0, s>>>(V, ldv, nv, w, n, k.h2, k.part, k.sc);
+    kry_givens_kernel<<<1, kKryThreads, 0, s>>>(H, ldh, cs, sn, g, k.h1, k.h2, k.sc, norm, B, j, inv_hn);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FRSDG_OK : report_cuda(e, "frsdg_gmres_arnoldi launch");
 }
