@@ -550,7 +550,7 @@ def run_ours(args, ws, rank, local):
     mean_launch_s = statistics.mean(launch_ms) / 1e3
     achieved = alg_bytes / mean_launch_s / 1e9
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic_per_launch(), "peak_kind": peak_kind, "kernel": "fr2d_kernel<double,6,VdW,HLLC,affine>",
+            "traffic": traffic_per_launch(), "peak_kind": peak_kind, "kernel": "fr2d_line_kernel<double,6,VdW,HLLC,affine>",
             "algorithmic_bytes_per_launch": alg_bytes, "mean_launch_ms": mean_launch_s * 1e3}
     # the FP64 compute bound beside it: operations of the reference algorithm per launch
     fl = flops_per_full_launch()

@@ -60,8 +60,8 @@ cudaError_t stage_launch(int n, int gas, int riem, int var, const Fr2dBatchArgs&
 // the single-instance kernels' shapes, variant 1 with half the rows.
 void residual_tile(int n, bool f32, int var, int* tx, int* ty)
 {
-    *tx = f32 ? tile_x(n, 1, true) : line_tile_x(n, false);
-    const int t = f32 ? tile_y(n, 1, true) : line_tile_y(n, false);
+    *tx = f32 ? tile_x(n, true) : line_tile_x(n, false);
+    const int t = f32 ? tile_y(n, true) : line_tile_y(n, false);
     *ty = var == 0 || t == 1 ? t : t / 2;
 }
 

@@ -1,4 +1,6 @@
-// residual2d.cuh -- fused FR residual of the 2D Euler equations.
+// residual2d.cuh -- fused FR residual of the 2D Euler equations: the complex-step product
+// (complex or dual scalars) and the mixed-form FP32 stages.  FP64 and FP32 states take one
+// thread per line of nodes instead (line2d.cuh).
 //
 // One CTA owns a tile of TX x TY elements and makes one pass over HBM:
 //   P1  every tile node: load (with the complex-step seed u + i h v or the
@@ -34,15 +36,11 @@ __host__ __device__ constexpr int round_up32(int v) { return (v + 31) / 32 * 32;
 // Block size and register cap of the 2D kernel (FRSDG_BT / FRSDG_MAXREG override
 // them for tuning builds).  A CTA's warps are spread over the SM's four
 // sub-partitions, each with a quarter of the register file.
-//   face tiles (FP64 at n >= 5, FP32 at n = 5 and 6): one thread per face point of the
-//     tile (x-face and y-face threads rounded to warps) plus one warp of element
-//     columns (two at n = 5), 80 registers, so that 4-6 CTAs share an SM;
+//   face tiles (FP32 at n = 5 and 6): one thread per face point of the tile (x-face and
+//     y-face threads rounded to warps) plus one warp of element columns (two at n = 5);
 //   otherwise: one thread per tile node (128 to 512), the cap chosen for three
 //     co-resident CTAs (one for complex).
-// Measured on B200 (1024^2 blast rhs, FP64): p = 4 1.56 -> 1.41 ms, p = 5 1.77 ->
-// 1.57 ms, p = 6 4.17 -> 2.91 ms, p = 7 3.48 -> 3.36 ms, p = 8 4.21 -> 3.82 ms,
-// p = 9 6.79 -> 4.68 ms; at p = 2 and 3 one thread per node stays ahead (0.52 and
-// 0.86 ms against 0.62 and 0.95).  FP32: p = 5 1.00 -> 0.96 ms; at p = 4 one thread
+// Measured on B200, FP32: p = 5 1.00 -> 0.96 ms (1024^2 blast); at p = 4 one thread
 // per node is ahead on the 1024^2 mesh (0.75 against 0.85 ms) but behind on the 64^2
 // curved vortex of the mixed-precision runs (0.27 against 0.18 s to t = 10), which
 // fills fewer than two waves of CTAs, so FP32 takes face tiles at p = 4 and 5.
@@ -50,12 +48,12 @@ __host__ __device__ constexpr int face_threads(int n, int tx, int ty)
 {
     return round_up32((tx + 1) * ty * n) + round_up32(tx * (ty + 1) * n);
 }
-__host__ __device__ constexpr int block_threads(int n, int words, bool f32, int tx, int ty)
+__host__ __device__ constexpr int block_threads(int n, bool f32, int tx, int ty)
 {
 #ifdef FRSDG_BT
     return FRSDG_BT;
 #else
-    if (face_tiles(n, words, f32)) return face_threads(n, tx, ty) + (n == 5 ? 64 : 32);
+    if (face_tiles(n, f32)) return face_threads(n, tx, ty) + (n == 5 ? 64 : 32);
     const int tile_nodes = tx * ty * n * n;
     return round_up32(tile_nodes > 128 ? (tile_nodes < 512 ? tile_nodes : 512) : 128);
 #endif
@@ -68,11 +66,11 @@ __host__ __device__ constexpr int reg_cap(int n, int words, bool f32, int bt)
     // FP32 at n = 6: 56 registers, six CTAs per SM despite some spills (1024^2 blast
     // 0.89 -> 0.84 ms); at n = 5 the same cap is faster on the 1024^2 mesh (0.79 -> 0.69
     // ms) but slower on the 64^2 curved vortex of the mixed-precision runs (0.18 -> 0.24 s
-    // to t = 10), so n = 5 keeps 80.  FP64: 80 registers, no spills.
+    // to t = 10), so n = 5 keeps 80.
 #ifndef FRSDG_F32_REG6
 #define FRSDG_F32_REG6 56
 #endif
-    if (face_tiles(n, words, f32)) return f32 && n == 6 ? FRSDG_F32_REG6 : 80;
+    if (face_tiles(n, f32)) return n == 6 ? FRSDG_F32_REG6 : 80;
     // three co-resident CTAs (one for complex): per sub-partition ceil(ctas*warps/4) warps
     return (16384 / (32 * (((words == 2 ? 1 : 3) * (bt / 32) + 3) / 4))) / 8 * 8;
 #endif
@@ -87,12 +85,12 @@ template <class S, int N, int GEO, int VAR = 0, bool TC = false> struct Tile2D
 {
     static constexpr int W  = scalar_traits<S>::words;
     static constexpr bool F32 = sizeof(S) == 4;
-    static constexpr int TX = tile_x(N, W, F32);
-    static constexpr int TY = VAR == 0 || tile_y(N, W, F32) == 1 ? tile_y(N, W, F32) : tile_y(N, W, F32) / 2;
+    static constexpr int TX = tile_x(N, F32);
+    static constexpr int TY = VAR == 0 || tile_y(N, F32) == 1 ? tile_y(N, F32) : tile_y(N, F32) / 2;
     static constexpr int NN = N * N;
     static constexpr int TE = TX * TY;
     static constexpr bool JVP = scalar_traits<S>::words == 2;
-    static constexpr int BT = block_threads(N, W, F32, TX, TY);
+    static constexpr int BT = block_threads(N, F32, TX, TY);
     // tensor-core tiles: shared memory admits four or five CTAs per SM, so 80 registers
 #ifdef FRSDG_TC_MAXREG
     static constexpr int MAXREG = TC ? FRSDG_TC_MAXREG : reg_cap(N, W, F32, BT) > 255 ? 255 : reg_cap(N, W, F32, BT);

@@ -9,9 +9,9 @@ module is the PETSc-free equivalent on the GPU:
 
   * J v       frsdg_jvp_prepare / frsdg_jvp (complex-step JVP kernel);
   * P^-1 r    frsdg_pc_setup / frsdg_pc_apply (element block-Jacobi: the diagonal
-              blocks of J from one coloured complex-step launch, FP32 inverses), or
+              blocks of J from one launch, FP32 inverses), or
               frsdg_pc_setup_gs (red-black block Gauss-Seidel over all five blocks of an
-              element row, from one distance-2 coloured launch);
+              element row, from one launch);
   * coarse    optional second level (CoarseCorrection): the Galerkin operator
               P^T J P on piecewise-constant aggregates of elements, probed with 20
               JVPs (aggregates coloured (I + 2J) mod 5, four variables), inverted
@@ -203,8 +203,7 @@ class CoarseCorrection:
     J couples an element to its face neighbours only, so J P couples an aggregate to
     its four face-neighbour aggregates: colouring the aggregates by (I + 2J) mod 5
     gives every closed five-aggregate neighbourhood distinct colours, and A_c follows
-    from 5 colours x 4 variables = 20 JVPs (the way the element blocks are probed by
-    frsdg_jac_blocks5).  A_c (4 * aggregates square, FP64) is inverted (or LU-factorised)
+    from 5 colours x 4 variables = 20 JVPs.  A_c (4 * aggregates square, FP64) is inverted (or LU-factorised)
     once per set-up; meshes of a few thousand aggregates keep it small."""
 
     def __init__(self, cfg: A.frsdg_config, ax: int = 4, ay: int = 4, explicit_inverse: bool = True):

@@ -139,7 +139,7 @@ class FRSolver:
         A.check(self._lib.frsdg_jvp(self._h, _ptr(v), _ptr(out), _stream()), "frsdg_jvp")
 
     def jac_blocks(self, t: float, sigma: float, U: torch.Tensor, blocks: torch.Tensor) -> None:
-        """Element-diagonal Jacobian blocks (coloured complex step), blocks[e] column-major."""
+        """Element-diagonal Jacobian blocks (complex step), blocks[e] column-major."""
         self._check_vec(U)
         nd = self.n_dofs // self.n_elems
         if blocks.dtype != torch.float64 or not blocks.is_cuda or not blocks.is_contiguous() \
@@ -153,7 +153,7 @@ class FRSolver:
         A.check(self._lib.frsdg_pc_setup(self._h, t, sigma, _ptr(U), _stream()), "frsdg_pc_setup")
 
     def jac_blocks5(self, t: float, sigma: float, U: torch.Tensor, blocks5: torch.Tensor) -> None:
-        """All five blocks of every element row (distance-2 coloured complex step)."""
+        """All five blocks of every element row (complex step)."""
         self._check_vec(U)
         nd = self.n_dofs // self.n_elems
         if blocks5.dtype != torch.float64 or not blocks5.is_cuda or not blocks5.is_contiguous() \

@@ -220,11 +220,10 @@ int frsdg_rk_stage_mixed(frsdg_handle* h, double t, const double* Us, const doub
  *   FRSDG_STAGE_POST_STEP  out = frsdg_post_step applied to out (the spectral filter of
  *                          cfg.apply_filter, then the limiter of cfg.pp_limit) -- the last
  *                          stage of a step.
- * With FRSDG_STAGE_POST_STEP in 2D, when the post-step is element-local (the filter,
- * the limiter, or nothing; not the WENO limiter alone, which reads neighbours), this is
- * ONE launch: each CTA finishes its elements' stage values in shared memory, filters
- * and limits them there and writes out once.  Otherwise (1D, WENO, and the limiter
- * alone, which is faster as its own pass) it runs the stage and then the separate
+ * An element-local post-step (the filter, the limiter, or nothing; not the WENO limiter
+ * alone, which reads neighbours) and the limiter of FRSDG_STAGE_LIMIT run in the stage's
+ * launch, on its values before they are written.  Otherwise (WENO, and the limiter alone
+ * after a mixed stage, which is faster as its own pass) the stage runs and then the separate
  * passes.  Results equal the unfused sequence's up to rounding.  out may alias A (the
  * state updated in place) but not Us. */
 enum { FRSDG_STAGE_MIXED = 1, FRSDG_STAGE_LIMIT = 2, FRSDG_STAGE_POST_STEP = 4 };
@@ -233,28 +232,26 @@ int frsdg_rk_stage_fused(frsdg_handle* h, double t, const double* Us, const doub
                          double delta, int32_t flags, void* stream);
 
 /* Element-diagonal blocks of the implicit Jacobian J = sigma*dM/dU + dR(M(U))/dU at
- * (t, U), by complex step (h = cfg.csd_eps) with element colouring, in one launch:
- * the preconditioner's part of ComplexStepJacobianStrategy::pre_jv_eval
- * (petsc_solver_impl.hpp:223-248), which assembles its preconditioner by DMDA-coloured
- * finite differences (MatFDColoringApply, 72-95, 244).  Elements of one colour share
- * no face, so seeding DOF d of every element of colour c gives column d of each such
- * element's block.  blocks: nelem * nd * nd doubles (nd = 4 (p+1)^2), block e
- * column-major: blocks[(e*nd + col)*nd + row].  2D only. */
+ * (t, U), by complex step (h = cfg.csd_eps), in one launch: the preconditioner's part of
+ * ComplexStepJacobianStrategy::pre_jv_eval (petsc_solver_impl.hpp:223-248), which
+ * assembles its preconditioner by DMDA-coloured finite differences (MatFDColoringApply,
+ * 72-95, 244).  The columns are assembled from the complex-step derivatives of the node
+ * and face fluxes and equal single-seed products of frsdg_jvp up to rounding.  blocks:
+ * nelem * nd * nd doubles (nd = 4 (p+1)^2), block e column-major:
+ * blocks[(e*nd + col)*nd + row].  2D only. */
 int frsdg_jac_blocks(frsdg_handle* h, double t, double sigma, const double* U,
                      double* blocks, void* stream);
 
 /* Block-Jacobi preconditioner for the Newton-Krylov solve (the PCSetUp / PCApply
- * pair PETSc runs on the coloured Jacobian): frsdg_pc_setup computes the blocks of
- * frsdg_jac_blocks into handle-owned storage (allocated by the first call:
- * nelem*nd*nd doubles and as many floats), inverts each block in FP64 with partial
- * pivoting, keeps the inverses in FP32, synchronises the stream and fails with
- * FRSDG_ERR_ARG on a zero pivot; p <= 5.  frsdg_pc_apply: z_e = inv(J_ee) r_e for
+ * pair PETSc runs on the coloured Jacobian): frsdg_pc_setup inverts the blocks of
+ * frsdg_jac_blocks in FP64 with partial pivoting, keeps the inverses in FP32 in
+ * handle-owned storage (nelem*nd*nd floats, allocated by the first call), synchronises
+ * the stream and fails with FRSDG_ERR_ARG on a zero pivot; p <= 5.  frsdg_pc_apply: z_e = inv(J_ee) r_e for
  * every element (z must not alias r). */
 int frsdg_pc_setup(frsdg_handle* h, double t, double sigma, const double* U, void* stream);
 
 /* All five blocks of every element row of the same Jacobian (the element and its four
- * face neighbours) from one complex-step launch with the distance-2 colouring
- * (i + 2 j) mod 5: blocks5: nelem * 5 * nd * nd doubles, block (e, s) column-major at
+ * face neighbours) from one launch: blocks5: nelem * 5 * nd * nd doubles, block (e, s) column-major at
  * ((e*5 + s)*nd + col)*nd + row, s = 0 self, 1 right, 2 top, 3 bottom, 4 left (zero where
  * the neighbour does not exist).  2D, whole mesh; periodic directions need a multiple of
  * 5 elements. */
@@ -262,9 +259,10 @@ int frsdg_jac_blocks5(frsdg_handle* h, double t, double sigma, const double* U,
                       double* blocks5, void* stream);
 
 /* Red-black block Gauss-Seidel preconditioner from those blocks (non-periodic 2D
- * meshes, p <= 5): frsdg_pc_setup_gs computes them into handle-owned storage (first call
- * allocates 5 nelem nd^2 doubles and 5 nelem nd^2 floats), inverts the diagonal blocks
- * (FP64, partial pivoting, kept in FP32), keeps the couplings in FP32 and makes
+ * meshes, p <= 5): frsdg_pc_setup_gs inverts the diagonal blocks (FP64, partial pivoting,
+ * kept in FP32), keeps the neighbours' couplings in FP32, nonzeros only (a row couples to
+ * one face node of each neighbour; the first call allocates nelem (nd^2 + 16 nd) floats),
+ * and makes
  * frsdg_pc_apply run one symmetric sweep: red z = D^-1 r; black z = D^-1 (r - J z_red);
  * red z -= D^-1 J z_black.  Synchronises the stream; FRSDG_ERR_ARG on a zero pivot. */
 int frsdg_pc_setup_gs(frsdg_handle* h, double t, double sigma, const double* U, void* stream);
@@ -387,8 +385,8 @@ int frsdg_batch_destroy(frsdg_batch* b);
  * PETSc, -ts_max_reject, tools/c-vcjh_test.py:100-105) reads both. */
 int frsdg_check_state(frsdg_handle* h, const double* U, void* stream);
 
-/* The library's device FP64 reciprocal (op 0) and square root (op 1) -- a
- * single-precision seed refined by Newton steps, used throughout the residual --
+/* The library's device FP64 reciprocal (op 0) and square root (op 1) -- the hardware's
+ * approximations refined to full precision, used throughout the residual --
  * applied elementwise to the device array x[0..n) into y, for validation against
  * IEEE division and sqrt.  Ops 2 and 3: the same in the deferred form of the residual's
  * node and face passes (the fast path, redone with ops 0 / 1 when the input lies
