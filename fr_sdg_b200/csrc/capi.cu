@@ -874,11 +874,17 @@ static int run_pc_setup(frsdg_handle* h, double t, double sigma, const double* U
     cudaError_t e;
     const size_t nb = size_t(h->nelem) * nd * nd, no = size_t(h->nelem) * size_t(offdiag_floats(nd));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (!h->d_inv)
+    if (!h->d_inv && (e = cudaMalloc(&h->d_inv, sizeof(float) * nb)) != cudaSuccess)
+        return cuda_fail(e, "cudaMalloc(inverse blocks)");
+    if (h->win_rows)
     {
-        if ((e = cudaMalloc(&h->d_inv, sizeof(float) * nb)) != cudaSuccess) return cuda_fail(e, "cudaMalloc(inverse blocks)");
-        // the ghost rows of a row window have no block: z = 0 there
-        if ((e = cudaMemsetAsync(h->d_inv, 0, sizeof(float) * nb, s)) != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
+        // the blocks stand at their elements' global rows; the rows outside a window have none:
+        // z = 0 there, whatever an earlier set-up left
+        const size_t row = size_t(h->Nx) * nd * nd;
+        const size_t g0 = size_t(h->win_base + h->win_begin), g1 = size_t(h->win_base + h->win_end);
+        if ((e = cudaMemsetAsync(h->d_inv, 0, sizeof(float) * row * g0, s)) != cudaSuccess ||
+            (e = cudaMemsetAsync(h->d_inv + row * g1, 0, sizeof(float) * row * (size_t(h->Ny) - g1), s)) != cudaSuccess)
+            return cuda_fail(e, "cudaMemsetAsync");
     }
     if (gs && !h->d_off && (e = cudaMalloc(&h->d_off, sizeof(float) * no)) != cudaSuccess)
         return cuda_fail(e, "cudaMalloc(blocks)");
@@ -929,8 +935,19 @@ int frsdg_pc_apply(frsdg_handle* h, const double* r, double* z, void* stream)
     if (r == z) return fail(FRSDG_ERR_ARG, "frsdg_pc_apply: z must not alias r");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     h->last = s;
-    const cudaError_t e = launch_pc_apply(h->d_inv, h->pc_kind == 2 ? h->d_off : nullptr, r, z, h->n, h->Nx,
-                                          h->win_rows ? h->win_rows : h->Ny, s);
+    cudaError_t e;
+    if (!h->win_rows)
+        e = launch_pc_apply(h->d_inv, h->pc_kind == 2 ? h->d_off : nullptr, r, z, h->n, h->Nx, h->Ny, s);
+    else
+    {
+        // the window's computed rows against the blocks of their global rows; ghost rows: z = 0
+        const size_t row = size_t(h->Nx) * h->ndofs, begin = size_t(h->win_begin), end = size_t(h->win_end);
+        const float* inv = h->d_inv + size_t(h->win_base + h->win_begin) * row * h->ndofs;
+        e = cudaMemsetAsync(z, 0, sizeof(double) * row * begin, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(z + row * end, 0, sizeof(double) * row * (size_t(h->win_rows) - end), s);
+        if (e == cudaSuccess)
+            e = launch_pc_apply(inv, nullptr, r + row * begin, z + row * begin, h->n, h->Nx, int(end - begin), s);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "block-apply launch");
     return FRSDG_OK;
 }

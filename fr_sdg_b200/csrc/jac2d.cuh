@@ -317,8 +317,8 @@ __global__ void __launch_bounds__(kJacThreads, Jac2D<N>::R <= 4 ? 3 : 1) jac2d_i
     int* pinv = perm + ND;                               // k of row r_k
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31;
     const int gi = int(blockIdx.x) % a.Nx, gj = a.row_begin + int(blockIdx.x) / a.Nx;
-    const int64_t e = int64_t(gj) * a.Nx + gi;
-    const int64_t mbase = (int64_t(gj + a.row_base) * a.Nx + gi) * NN;
+    const int64_t e = int64_t(gj + a.row_base) * a.Nx + gi;  // by global row: any window's rows fit the mesh's storage
+    const int64_t mbase = e * NN;
     jac_derivatives<C, N, GAS, RIEM>(a, gi, gj, sm);
     if (off)
         for (int q = tid; q < 4 * NN; q += kJacThreads)

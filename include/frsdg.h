@@ -247,7 +247,8 @@ int frsdg_jac_blocks(frsdg_handle* h, double t, double sigma, const double* U,
  * frsdg_jac_blocks in FP64 with partial pivoting, keeps the inverses in FP32 in
  * handle-owned storage (nelem*nd*nd floats, allocated by the first call), synchronises
  * the stream and fails with FRSDG_ERR_ARG on a zero pivot; p <= 5.  frsdg_pc_apply: z_e = inv(J_ee) r_e for
- * every element (z must not alias r). */
+ * every element (z must not alias r).  With a row window the set-up takes the window's
+ * computed rows, and z is zero in ghost rows and in rows that the last set-up left out. */
 int frsdg_pc_setup(frsdg_handle* h, double t, double sigma, const double* U, void* stream);
 
 /* All five blocks of every element row of the same Jacobian (the element and its four
