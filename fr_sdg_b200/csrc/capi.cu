@@ -933,6 +933,8 @@ int frsdg_pc_apply(frsdg_handle* h, const double* r, double* z, void* stream)
     if (!h || !r || !z) return fail(FRSDG_ERR_ARG, "null argument");
     if (!h->pc_kind) return fail(FRSDG_ERR_ARG, "frsdg_pc_apply called before frsdg_pc_setup");
     if (r == z) return fail(FRSDG_ERR_ARG, "frsdg_pc_apply: z must not alias r");
+    if (h->pc_kind == 2 && h->win_rows)
+        return fail(FRSDG_ERR_UNSUPPORTED, "frsdg_pc_apply: the Gauss-Seidel sweep takes the whole mesh (no row window)");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     h->last = s;
     cudaError_t e;

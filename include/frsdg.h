@@ -265,7 +265,8 @@ int frsdg_jac_blocks5(frsdg_handle* h, double t, double sigma, const double* U,
  * one face node of each neighbour; the first call allocates nelem (nd^2 + 16 nd) floats),
  * and makes
  * frsdg_pc_apply run one symmetric sweep: red z = D^-1 r; black z = D^-1 (r - J z_red);
- * red z -= D^-1 J z_black.  Synchronises the stream; FRSDG_ERR_ARG on a zero pivot. */
+ * red z -= D^-1 J z_black (whole mesh: under a row window set-up and sweep are refused with
+ * FRSDG_ERR_UNSUPPORTED).  Synchronises the stream; FRSDG_ERR_ARG on a zero pivot. */
 int frsdg_pc_setup_gs(frsdg_handle* h, double t, double sigma, const double* U, void* stream);
 int frsdg_pc_apply(frsdg_handle* h, const double* r, double* z, void* stream);
 

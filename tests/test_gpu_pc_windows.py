@@ -80,3 +80,18 @@ def test_blocks_under_a_window(p, cuda):
             W = torch.empty(NX * rows * nd * nd, dtype=torch.float64, device=cuda)
             s.jac_blocks(0.0, 3.0, U.view(NY, row)[glob].reshape(-1), W)
             assert torch.equal(W.view(rows, row * nd)[begin:end], B[glob[begin:end]])
+
+
+def test_gauss_seidel_sweep_refuses_a_window(cuda):
+    """A sweep over a window's rows would take other elements' blocks."""
+    cfg = make_config(dim=2, p=2, n_elems=(NX, NY), riemann="hllc", csd_eps=1e-30,
+                      bcs={f: A.BC_OUTFLOW for f in (A.LEFT, A.RIGHT, A.TOP, A.BOTTOM)})
+    U = torch.from_numpy(random_state(cfg, 2, amp=0.2)).to(cuda)
+    with FRSolver(cfg) as s:
+        s.pc_setup_gs(0.0, 50.0, U)
+        s.set_row_window(2, 4, 1, 4)
+        r = torch.zeros(s.n_dofs, dtype=torch.float64, device=cuda)
+        with pytest.raises(A.FrsdgError):
+            s.pc_apply(r, torch.empty_like(r))
+        s.set_row_window(0, 0, 0, 0)
+        s.pc_apply(U, torch.empty_like(U))
