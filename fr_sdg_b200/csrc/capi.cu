@@ -581,7 +581,15 @@ namespace
 // rounding run on values and derivatives (dual): the same results with half the arithmetic
 // (256 x 64 bump, p = 3, h = 1e-30: a product 47 -> 36 us, five blocks per element 1.71 -> 0.77 ms).  At the reference's h = 1e-7
 // smooth_abs, whose eps is 1e-7 too, feels the step, so those stay complex.
+// The step of a dual seed is the power of two at or below h: the products of that step, with
+// nothing rounded in the seed and in the quotient by it.
 bool first_order(double h) { return h <= 1e-20; }
+double dual_step(double h)
+{
+    int e;
+    std::frexp(h, &e);
+    return std::ldexp(1.0, e - 1);
+}
 
 // post: 1D stages, the epilogue's part of the post-step (POST_*)
 int run_residual(frsdg_handle* h, int mode, double t, const double* U, const double* W, double* out, void* stream,
@@ -611,7 +619,8 @@ int run_residual(frsdg_handle* h, int mode, double t, const double* U, const dou
         apply_window(h, a);
         if (mode == MODE_JVP && first_order(hh))
         {
-            a.h = a.inv_h = 1.0;
+            a.h = dual_step(hh);
+            a.inv_h = 1.0 / a.h;
             e = dispatch2d<dual>(h->n, h->cfg.gas_law, h->cfg.riemann, h->geo, a, s);
         }
         else if (mode == MODE_JVP) e = dispatch2d<cplx>(h->n, h->cfg.gas_law, h->cfg.riemann, h->geo, a, s);
@@ -831,12 +840,11 @@ static int run_jac(frsdg_handle* h, double t, double sigma, const double* U, con
     a.t = t;
     a.cond_sys = h->cfg.cond_sys;
     a.U = U;
-    a.h = h->cfg.csd_eps;
-    a.inv_h = 1.0 / h->cfg.csd_eps;
+    const bool fo = first_order(h->cfg.csd_eps);
+    a.h = fo ? dual_step(h->cfg.csd_eps) : h->cfg.csd_eps;
+    a.inv_h = 1.0 / a.h;
     a.sigma = sigma;
     apply_window(h, a);
-    const bool fo = first_order(h->cfg.csd_eps);
-    if (fo) a.h = a.inv_h = 1.0;
     const cudaError_t e = fo ? dispatch_jac2d<dual>(h->n, h->cfg.gas_law, h->cfg.riemann, a, o, s)
                              : dispatch_jac2d<cplx>(h->n, h->cfg.gas_law, h->cfg.riemann, a, o, s);
     if (e != cudaSuccess) return cuda_fail(e, "Jacobian-block launch");

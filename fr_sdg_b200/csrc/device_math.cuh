@@ -3,8 +3,8 @@
 // The residual is templated on its scalar S:
 //   double  the FP64 residual (rhs_func / fun_implicit),
 //   cplx    complex FP64 for the complex-step JVP (matmult of the reference),
-//   dual    value and directional derivative in FP64: the complex step's limit h -> 0, which
-//           takes the place of cplx when h^2 is below rounding (csd_eps <= 1e-20);
+//   dual    complex FP64 to first order in the imaginary part, which takes the place of cplx
+//           when h^2 is below rounding (csd_eps <= 1e-20);
 //   float   the FP32 residual of the mixed-precision form.
 // cplx follows std::complex<double> semantics for finite values: principal-branch
 // sqrt, Smith's division (R. L. Smith, "Algorithm 116: Complex division",
@@ -55,8 +55,10 @@ __device__ __forceinline__ cplx operator/(double s, cplx b) { return cplx(s) / b
 __device__ __forceinline__ cplx& operator+=(cplx& a, cplx b) { a = a + b; return a; }
 __device__ __forceinline__ cplx& operator-=(cplx& a, cplx b) { a = a - b; return a; }
 
-// Value and derivative (re, im as in cplx): the products' second-order terms, h^2 smaller
-// than the first-order ones, are left out, and a quotient needs one reciprocal.
+// A complex number with an imaginary part of order h, |h| <= 1e-20 (the step is in im, as in
+// cplx): the products' second-order terms, h^2 smaller than the first-order ones, are left
+// out, and a quotient needs one reciprocal.  As in cplx the imaginary part decides where the
+// real one is zero, and the root of a negative value stands in the imaginary part.
 struct __align__(16) dual
 {
     double re, im;
@@ -138,7 +140,7 @@ __device__ __forceinline__ cplx s_sqrt(cplx z)
     if (z.re >= 0.0) return {t, z.im / (2.0 * t)};
     return {fabs(z.im) / (2.0 * t), copysign(t, z.im)};
 }
-// as the complex root to first order: principal branch, 0 at 0
+// Outside the fast range: the complex root, principal branch, to first order in the smaller part.
 __device__ __forceinline__ dual s_sqrt(dual z)
 {
     if (positive_in_float_range(z.re))
@@ -147,14 +149,13 @@ __device__ __forceinline__ dual s_sqrt(dual z)
         const double g = sqrt_fast(z.re, h);
         return {g, z.im * h};
     }
-    if (z.re == 0.0 && z.im == 0.0) return {0.0, z.im};
-    const double t = ieee_sqrt(fabs(z.re));
-    if (z.re >= 0.0) return {t, z.im / (2.0 * t)};
-    return {fabs(z.im) / (2.0 * t), copysign(t, z.im)};
+    const double t = ieee_sqrt(z.re == 0.0 ? 0.5 * fabs(z.im) : fabs(z.re));
+    if (t == 0.0) return {0.0, z.im};
+    const double q = z.im / (2.0 * t);
+    return z.re < 0.0 ? dual(fabs(q), copysign(t, z.im)) : dual(t, q);
 }
 __device__ __forceinline__ double s_log(double x) { return log(x); }
 __device__ __forceinline__ cplx s_log(cplx z) { return {log(hypot(z.re, z.im)), atan2(z.im, z.re)}; }
-__device__ __forceinline__ dual s_log(dual z) { return {log(z.re), z.im / z.re}; }
 __device__ __forceinline__ double s_exp(double x) { return exp(x); }
 __device__ __forceinline__ dual s_exp(dual z)
 {
@@ -190,16 +191,14 @@ __device__ __forceinline__ float s_rcp(float x) { return 1.0f / x; }
 __device__ __forceinline__ cplx s_rcp(cplx z) { return cplx(1.0) / z; }
 __device__ __forceinline__ dual s_rcp(dual z)
 {
-    const double r = s_rcp(z.re);
-    return {r, -(z.im * r) * r};
+    if (in_float_range(z.re))
+    {
+        const double r = rcp_fast(z.re);
+        return {r, -(z.im * r) * r};
+    }
+    const double r = ieee_rcp(z.re == 0.0 ? z.im : z.re);
+    return z.re == 0.0 ? dual(0.0, -r) : dual(r, -(z.im * r) * r);
 }
-__device__ __forceinline__ dual operator/(dual a, dual b)
-{
-    const double q = a.re / b.re;
-    return {q, (a.im - q * b.im) / b.re};
-}
-__device__ __forceinline__ dual operator/(dual a, double s) { return {a.re / s, a.im / s}; }
-__device__ __forceinline__ dual operator/(double s, dual b) { return dual(s) / b; }
 
 // wrap_positive (macro_and_libc.hpp:117-138): max(DBL_MIN, rho); for complex, the
 // real part decides and a clamped value loses its imaginary part.
@@ -302,7 +301,7 @@ __device__ __forceinline__ double s_re(cplx z) { return z.re; }
 __device__ __forceinline__ double s_im(cplx z) { return z.im; }
 __device__ __forceinline__ double s_re(dual z) { return z.re; }
 __device__ __forceinline__ double s_im(dual z) { return z.im; }
-__device__ __forceinline__ double s_branch(dual z) { return z.re; }
+__device__ __forceinline__ double s_branch(dual z) { return z.re + z.im; }
 __device__ __forceinline__ double s_branch(double x) { return x; }
 __device__ __forceinline__ double s_branch(float x) { return x; }
 __device__ __forceinline__ double s_branch(cplx z) { return z.re + z.im; }

@@ -298,6 +298,7 @@ __device__ __forceinline__ void riemann_rec(const S L[RF_N], const S R[RF_N], do
     {
         const S sL = smooth_min(unL - cL, unR - cR, m);
         const S sR = smooth_max(unL + cL, unR + cR, m);
+        const bool takeL = s_branch(sL) >= 0.0, rightR = s_branch(sR) >= 0.0;
         const S rhoL_diff = L[RF_RHO] * (sL - unL);
         const S rhoR_diff = R[RF_RHO] * (sR - unR);
         const S sM = (pR - pL + unL * rhoL_diff - unR * rhoR_diff) * m.rcp(rhoL_diff - rhoR_diff);
@@ -315,8 +316,7 @@ __device__ __forceinline__ void riemann_rec(const S L[RF_N], const S R[RF_N], do
         const S st1 = (sM * (sK * (K0 * unK) - FK1) + sK * p_star) * inv;
         const S st2 = utK * st0;
         const S st3 = (sM * (sK * K3 - FK3) + sK * p_star * sM) * inv;
-        const bool takeL = s_branch(sL) >= 0.0;
-        const bool star  = left || s_branch(sR) >= 0.0;
+        const bool star  = left || rightR;
         f0 = takeL ? FL0 : (star ? st0 : FR0);
         f1 = takeL ? FL1 : (star ? st1 : FR1);
         f2 = takeL ? FL2 : (star ? st2 : FR2);
@@ -556,15 +556,13 @@ __device__ __forceinline__ void bc_ghost2(const BcDev& b, int dir, const GasPara
 {
     if constexpr (std::is_same<S, dual>::value)
     {
-        // the complex formulas with a step whose square is far below rounding
-        constexpr double h = 1e-30;
         if (exact)
         {
             cplx ci[4], co[4];
-            for (int q = 0; q < 4; ++q) ci[q] = cplx(in[q].re, in[q].im * h);
+            for (int q = 0; q < 4; ++q) ci[q] = cplx(in[q].re, in[q].im);
             if (bc_ghost2_exact<GAS>(b, g, nx, ny, ci, co))
             {
-                for (int q = 0; q < 4; ++q) out[q] = S(co[q].re, co[q].im * 1e30);
+                for (int q = 0; q < 4; ++q) out[q] = S(co[q].re, co[q].im);
                 return;
             }
         }

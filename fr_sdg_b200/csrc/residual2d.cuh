@@ -185,7 +185,7 @@ template <> struct NodeLoader<float>
     }
 };
 
-// the complex-step point u + i h v (dual: h = 1)
+// the complex-step point u + i h v
 template <class C> struct ComplexLoader
 {
     __device__ static void load(const Fr2dArgs& a, int64_t off, C s[4])

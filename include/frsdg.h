@@ -183,7 +183,9 @@ int frsdg_ifunction(frsdg_handle* h, double t, const double* U, const double* U_
 int frsdg_jvp_prepare(frsdg_handle* h, double t, double sigma, const double* U);
 
 /* JV = sigma*Im(M(U+ihV))/h + Im(R(M(U+ihV)))/h, h = cfg.csd_eps:
- * ComplexStepJacobianStrategy::matmult (petsc_solver_impl.hpp:250-432). */
+ * ComplexStepJacobianStrategy::matmult (petsc_solver_impl.hpp:250-432).  In 2D at
+ * csd_eps <= 1e-20 h is the power of two at or below it and terms of order h^2, far below
+ * rounding, are left out. */
 int frsdg_jvp(frsdg_handle* h, const double* V, double* JV, void* stream);
 
 /* Row window for domain decomposition (2D; the reference's DMDA ghosted local view,
