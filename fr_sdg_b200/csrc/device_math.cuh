@@ -270,9 +270,10 @@ struct MathDeferred
         if (!positive_in_float_range(x)) bad = 1u;
         return sqrt_fast(x);
     }
-    // FP32: the hardware approximations with one Newton step (within 2 ulp of the IEEE
-    // results) for normal inputs whose results stay normal; zero, subnormals, huge values,
-    // inf and NaN (exponent tests as above) take the redo with the IEEE operations
+    // FP32: the hardware approximations with one Newton step for normal inputs whose results
+    // stay normal (equal to the IEEE results on every mantissa, so a redo of nodes that need
+    // none leaves their bits); zero, subnormals, huge values, inf and NaN (exponent tests as
+    // above) take the redo with the IEEE operations
     __device__ __forceinline__ float rcp(float x) const
     {
         const unsigned e = (__float_as_uint(x) >> 23) & 0xffu;
