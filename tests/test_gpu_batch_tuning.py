@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 def test_limited_batches_are_timed_by_themselves(cuda):
     times = []
     for limit in (False, True, False):
-        wl = circular_explosion((90, 70), 4, "ideal", 1.4, (0.0, 0.0), 0.25, 0.1)
+        wl = circular_explosion(77, 4, "ideal", 1.4, (0.0, 0.0), 0.25, 0.1)
         wl.cfg.pp_limit = int(limit)
         with FRSolver(wl.cfg) as s:
             U = wl.init(cuda)
