@@ -65,14 +65,15 @@ void residual_tile(int n, bool f32, int var, int* tx, int* ty)
     *ty = var == 0 || t == 1 ? t : t / 2;
 }
 
-// Autotuner choices, per (device, order, gas, flux, precision, tile count rounded up to a
-// power of two).
+// Autotuner choices, per (device, order, gas, flux, precision, limiter in the FP64 stages,
+// tile count rounded up to a power of two).
 struct TuneKey
 {
-    int dev, n, gas, riem, mixed, tiles_pow2;
+    int dev, n, gas, riem, mixed, limit, tiles_pow2;
     bool operator<(const TuneKey& o) const
     {
-        return std::tie(dev, n, gas, riem, mixed, tiles_pow2) < std::tie(o.dev, o.n, o.gas, o.riem, o.mixed, o.tiles_pow2);
+        return std::tie(dev, n, gas, riem, mixed, limit, tiles_pow2) <
+               std::tie(o.dev, o.n, o.gas, o.riem, o.mixed, o.limit, o.tiles_pow2);
     }
 };
 struct TuneChoice
@@ -250,7 +251,7 @@ int autotune(frsdg_batch* b, cudaStream_t s)
             while (v < g.ntiles[0]) v <<= 1;
             return v;
         }();
-        const TuneKey key{b->device, g.n, g.gas, g.riem, b->mixed, p2};
+        const TuneKey key{b->device, g.n, g.gas, g.riem, b->mixed, stage_args(b, g, 0, 0).limit, p2};
         bool cached = false;
         {
             std::lock_guard<std::mutex> lk(g_tune_mu);
