@@ -8,8 +8,9 @@
 //   1. rho_min < eps:  rho <- rho_bar + theta1 (rho - rho_bar),
 //                      theta1 = (rho_bar - eps) / (rho_bar - rho_min);
 //   2. U <- Ubar + theta2 (U - Ubar), theta2 = min over nodes with p < eps of the
-//      point t of the segment Ubar -> U_q with pressure eps (60 bisection steps,
-//      keeping the admissible end).
+//      point t of the segment Ubar -> U_q with pressure eps (Newton's iteration on a
+//      polynomial of t, its root moved to the admissible side; bisection where rho or
+//      1 - b rho is not positive along the segment).
 // It has no counterpart in the reference.  The argument type PA provides gas_law, gas,
 // eps0, w[] (GLL weights) and detJ (per-node Jacobian determinants, or null).
 #pragma once
@@ -94,16 +95,23 @@ template <class PA> __device__ __forceinline__ double node_wave_speed_fast(const
     return s_sqrt(v2) + s_sqrt(fmax(c2, 0.0));
 }
 
-// pp_pressure with reciprocals
-template <int NV, class PA> __device__ __forceinline__ double pp_pressure_rcp(const PA& a, const double* u)
+// The 1D screen: whether rho and p stand above thr whichever way p is rounded.  p from
+// reciprocals, and a margin of 16 roundings of the terms it is the difference of, well above
+// what this form and pp_pressure's quotients may differ by (4 roundings for an ideal gas).
+template <int NV, class PA> __device__ __forceinline__ bool pp_clear(const PA& a, const double* u, double thr)
 {
     double m2 = 0.0;
 #pragma unroll
     for (int c = 1; c < NV - 1; ++c) m2 += u[c] * u[c];
-    const double rho_e = u[NV - 1] - 0.5 * m2 * s_rcp(u[0]);
-    if (a.gas_law == FRSDG_GAS_IDEAL) return (a.gas.gamma - 1.0) * rho_e;
-    const double arr = a.gas.a * u[0] * u[0];
-    return ((a.gas.gamma - 1.0) * (rho_e + arr)) * s_rcp(1.0 - a.gas.b * u[0]) - arr;
+    const double k = a.gas.gamma - 1.0, kin = 0.5 * m2 * s_rcp(u[0]);
+    double p = k * (u[NV - 1] - kin), terms = k * (fabs(u[NV - 1]) + fabs(kin));
+    if (a.gas_law != FRSDG_GAS_IDEAL)
+    {
+        const double arr = a.gas.a * u[0] * u[0], ic = s_rcp(1.0 - a.gas.b * u[0]);
+        p = (p + k * arr) * ic - arr;
+        terms = (terms + k * arr) * fabs(ic) * (1.0 + fabs(ic)) + arr;  // 1 - b rho rounds by 1 / |1 - b rho|
+    }
+    return u[0] > thr && p > thr + 0x1p-49 * terms;
 }
 
 template <int NV> struct PPState
@@ -361,14 +369,15 @@ __device__ __forceinline__ void pp_element2d(const PA& a, double* base, float* b
 // One element of a 1D state ([eq][node]), limited by one thread.
 template <int N, class PA> __device__ __forceinline__ void pp_element1d(const PA& a, double* u)
 {
-    // elements whose nodes all have density and pressure above the floor stay as they are
+    // elements whose nodes all have density and pressure above the floor stay as they are; nodes
+    // within rounding of it are decided by pp_pressure below
     const double thr = a.eps0 * (1.0 + 1e-10);
     bool clear = true;
 #pragma unroll
     for (int q = 0; q < N; ++q)
     {
         const double uq[3] = {u[q], u[N + q], u[2 * N + q]};
-        clear = clear && uq[0] > thr && pp_pressure_rcp<3>(a, uq) > thr;
+        clear = clear && pp_clear<3>(a, uq, thr);
     }
     if (clear) return;
     double wsum = 0.0, ub[3] = {0.0, 0.0, 0.0};
