@@ -21,17 +21,77 @@ namespace frsdg
 namespace
 {
 
+// z_e = inv_e r_e for every element.  Four threads per node: thread (part, node) takes the
+// columns j = part mod 4 of the node's four rows (16 bytes of each column, an element's
+// threads whole columns), and the four sums meet in shared memory.  One thread per node read
+// the large meshes as fast, but on meshes that live in L2 its chain of ND columns set the
+// time: 16 x 16 elements, p = 3, 4, 5 10.4, 14.0, 18.6 -> 4.3, 4.9, 6.4 us; 64 x 64 elements
+// (67 to 340 MB of inverses from memory) 31.7, 51.3, 79.8 -> 22.4, 40.9, 71.7 us.
+template <int N> struct Apply
+{
+    static constexpr int NN = N * N, ND = 4 * NN, TPE = 4 * NN;          // threads per element
+    static constexpr int EPC = TPE <= 64 ? 128 / TPE : 1;                 // elements per CTA
+    static constexpr int THREADS = (EPC * TPE + 31) / 32 * 32;
+};
+template <int N>
+__global__ void __launch_bounds__(Apply<N>::THREADS) block_apply_kernel(const float* __restrict__ inv, const double* __restrict__ r,
+                                                                        double* __restrict__ z, int64_t nelem)
+{
+    using P = Apply<N>;
+    constexpr int NN = P::NN, ND = P::ND;
+    __shared__ __align__(16) double st[P::EPC][ND];
+    __shared__ __align__(16) double sp[P::EPC][3][ND];
+    const int slot = threadIdx.x / P::TPE, t = threadIdx.x - slot * P::TPE, part = t / NN, node = t - part * NN;
+    const int64_t e = int64_t(blockIdx.x) * P::EPC + slot;
+    const bool active = slot < P::EPC && e < nelem;
+    if (active) st[slot][t] = r[e * ND + t];
+    const float4* B = reinterpret_cast<const float4*>(inv + e * (int64_t(ND) * ND)) + node + part * NN;
+    __syncthreads();
+    double o[4] = {0.0, 0.0, 0.0, 0.0};
+    if (active)
+    {
+        constexpr int U = NN % 9 == 0 ? 9 : NN % 5 == 0 ? 5 : NN < 8 ? NN : 8;  // columns in flight
+        static_assert(NN % U == 0, "whole groups of columns");
+#pragma unroll
+        for (int j = 0; j < NN; j += U)
+        {
+            float4 b[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) b[q] = __ldg(B + (j + q) * 4 * NN);
+#pragma unroll
+            for (int q = 0; q < U; ++q)
+            {
+                const double v = st[slot][(j + q) * 4 + part];
+                o[0] = fma(static_cast<double>(b[q].x), v, o[0]);
+                o[1] = fma(static_cast<double>(b[q].y), v, o[1]);
+                o[2] = fma(static_cast<double>(b[q].z), v, o[2]);
+                o[3] = fma(static_cast<double>(b[q].w), v, o[3]);
+            }
+        }
+        if (part > 0)
+        {
+            double2* s = reinterpret_cast<double2*>(&sp[slot][part - 1][node * 4]);
+            s[0] = make_double2(o[0], o[1]);
+            s[1] = make_double2(o[2], o[3]);
+        }
+    }
+    __syncthreads();
+    if (!active || part > 0) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        z[e * ND + node * 4 + q] = (o[q] + sp[slot][0][node * 4 + q]) + (sp[slot][1][node * 4 + q] + sp[slot][2][node * 4 + q]);
+}
+
 constexpr int kSweepThreads = 256;
 enum Sweep : int
 {
-    SWEEP_ALL = 0,   // every element: z = inv r
     SWEEP_RED = 1,   // red elements: z = inv r
     SWEEP_BLACK = 2, // black elements: z = inv (r - J z)
     SWEEP_BACK = 3   // red elements: z -= inv (J z)
 };
 
 // One pass over the elements of a colour (the k-th element of a colour sits in row
-// k / ceil(Nx/2)) or over all.  One thread per node: its four rows of the column-major
+// k / ceil(Nx/2)).  One thread per node: its four rows of the column-major
 // FP32 inverse are 16 bytes of each column, so an element's threads read whole columns,
 // kUnroll columns in flight.  A neighbour couples to the node's rows through the four
 // variables of one of its face nodes (jac2d.cuh), 64 bytes of `off` per neighbour and
@@ -48,18 +108,9 @@ __global__ void __launch_bounds__(kSweepThreads) block_sweep_kernel(const float*
     __shared__ __align__(16) double st[EPC][ND];
     const int slot = threadIdx.x / NN, node = threadIdx.x - slot * NN;
     const int64_t k = int64_t(blockIdx.x) * EPC + slot;
-    int gi, gj;
-    if constexpr (PHASE == SWEEP_ALL)
-    {
-        gj = int(k / Nx);
-        gi = int(k - int64_t(gj) * Nx);
-    }
-    else
-    {
-        const int half = (Nx + 1) / 2;
-        gj = int(k / half);
-        gi = 2 * int(k - int64_t(gj) * half) + ((gj + (PHASE == SWEEP_BLACK ? 1 : 0)) & 1);
-    }
+    const int half = (Nx + 1) / 2;
+    const int gj = int(k / half);
+    const int gi = 2 * int(k - int64_t(gj) * half) + ((gj + (PHASE == SWEEP_BLACK ? 1 : 0)) & 1);
     const bool active = slot < EPC && gj < Ny && gi < Nx;
     const int64_t e = int64_t(gj) * Nx + gi;
     const int64_t row = e * ND + node * 4;
@@ -123,7 +174,7 @@ template <int N, int PHASE>
 cudaError_t sweep(const float* inv, const float* off, const double* r, double* z, int Nx, int Ny, cudaStream_t s)
 {
     constexpr int EPC = kSweepThreads / (N * N);
-    const int64_t slots = int64_t(PHASE == SWEEP_ALL ? Nx : (Nx + 1) / 2) * Ny;  // element slots of the pass
+    const int64_t slots = int64_t((Nx + 1) / 2) * Ny;  // element slots of the pass
     block_sweep_kernel<N, PHASE><<<unsigned((slots + EPC - 1) / EPC), kSweepThreads, 0, s>>>(
         inv, reinterpret_cast<const float4*>(off), r, z, Nx, Ny);
     return cudaGetLastError();
@@ -132,7 +183,13 @@ cudaError_t sweep(const float* inv, const float* off, const double* r, double* z
 template <int N>
 cudaError_t apply_n(const float* inv, const float* off, const double* r, double* z, int Nx, int Ny, cudaStream_t s)
 {
-    if (!off) return sweep<N, SWEEP_ALL>(inv, off, r, z, Nx, Ny, s);
+    if (!off)
+    {
+        using P = Apply<N>;
+        const int64_t nelem = int64_t(Nx) * Ny;
+        block_apply_kernel<N><<<unsigned((nelem + P::EPC - 1) / P::EPC), P::THREADS, 0, s>>>(inv, r, z, nelem);
+        return cudaGetLastError();
+    }
     cudaError_t e;
     if ((e = sweep<N, SWEEP_RED>(inv, off, r, z, Nx, Ny, s)) != cudaSuccess) return e;
     if ((e = sweep<N, SWEEP_BLACK>(inv, off, r, z, Nx, Ny, s)) != cudaSuccess) return e;
