@@ -58,7 +58,11 @@ __device__ __forceinline__ cplx& operator-=(cplx& a, cplx b) { a = a - b; return
 // A complex number with an imaginary part of order h, |h| <= 1e-20 (the step is in im, as in
 // cplx): the products' second-order terms, h^2 smaller than the first-order ones, are left
 // out, and a quotient needs one reciprocal.  As in cplx the imaginary part decides where the
-// real one is zero, and the root of a negative value stands in the imaginary part.
+// real one is zero, and the root of a negative value stands in the imaginary part.  The real
+// parts round as cplx's do (a product of two by itself, not fused with a sum beside it): where
+// two wave speeds are equal but for rounding, smooth_abs divides that by its 1e-7, and other
+// roundings give other derivatives (bump channel: a product's distance to a complex FP64
+// restatement 1e-15 fused, 4e-16 so, in the same time).
 struct __align__(16) dual
 {
     double re, im;
@@ -69,7 +73,7 @@ struct __align__(16) dual
 __device__ __forceinline__ dual operator+(dual a, dual b) { return {a.re + b.re, a.im + b.im}; }
 __device__ __forceinline__ dual operator-(dual a, dual b) { return {a.re - b.re, a.im - b.im}; }
 __device__ __forceinline__ dual operator-(dual a) { return {-a.re, -a.im}; }
-__device__ __forceinline__ dual operator*(dual a, dual b) { return {a.re * b.re, fma(a.re, b.im, a.im * b.re)}; }
+__device__ __forceinline__ dual operator*(dual a, dual b) { return {__dmul_rn(a.re, b.re), fma(a.re, b.im, a.im * b.re)}; }
 __device__ __forceinline__ dual operator*(double s, dual a) { return {s * a.re, s * a.im}; }
 __device__ __forceinline__ dual operator*(dual a, double s) { return {a.re * s, a.im * s}; }
 __device__ __forceinline__ dual operator+(dual a, double s) { return {a.re + s, a.im}; }

@@ -192,7 +192,7 @@ __device__ __forceinline__ dual pmul(dual a, dual b)
 }
 __device__ __forceinline__ dual pfma(dual a, dual b, dual c)
 {
-    return {fma(a.re, b.re, c.re), fma(a.re, b.im, fma(a.im, b.re, c.im))};
+    return {__dmul_rn(a.re, b.re) + c.re, fma(a.re, b.im, fma(a.im, b.re, c.im))};
 }
 __device__ __forceinline__ double pfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float pfma(float a, float b, float c) { return fmaf(a, b, c); }

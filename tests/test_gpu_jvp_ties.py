@@ -81,3 +81,36 @@ def test_inadmissible_node_is_not_plausible(cuda):
         s.matmult(torch.from_numpy(V).to(cuda), out)
         got = float(out.abs().max())
     assert ref > 1e20 and not got < 1e20  # NaN counts as not plausible too
+
+
+@pytest.mark.parametrize("flow", ["tangential", "isothermal"])
+@pytest.mark.parametrize("p", [2, 3, 4])
+def test_real_parts_round_as_complex_ones(p, flow, cuda):
+    """Velocities along the y-faces of a curved mesh but for 1e-7, or one temperature and velocity at
+    random densities: smooth_abs divides the rounding of the normal velocity, or of the
+    difference of two equal wave speeds, by its 1e-7.  The first-order form has the complex form's
+    real parts, but for one reciprocal in 3000 and one root in 25 (the complex root takes a
+    hypot, which is not correctly rounded): an entry meets up to four face points, so most
+    entries of the two differ by the rounding of their imaginary parts alone, a few units of
+    2^-53 of their terms."""
+    def product(h):
+        cfg = make_config(dim=2, p=p, n_elems=(7, 6), box=(1.0, 1.0), riemann="rusanov", csd_eps=h,
+                          geometry=A.GEOM_SINE_WARP, geom_params=(0.05, 0, 0, 0),
+                          bcs={f: A.BC_PERIODIC for f in (A.LEFT, A.RIGHT, A.TOP, A.BOTTOM)})
+        ex, ey = Oracle(cfg).node_metrics()[:, 2:4].T
+        rng = np.random.default_rng(p)
+        r = rng.uniform(-1, 1, (ex.size, 4))
+        rho, pr, l = 1.0 + 0.1 * r[:, 0], 1.0 + 0.1 * r[:, 1], np.hypot(ex, ey)
+        u, v = 0.5 * ey / l + 1e-7 * r[:, 2], -0.5 * ex / l + 1e-7 * r[:, 3]
+        if flow == "isothermal":
+            pr, u, v = rho, np.full_like(u, 0.5), np.full_like(v, 0.3)
+        U = np.stack([rho, rho * u, rho * v, pr / 0.4 + 0.5 * rho * (u * u + v * v)], axis=1).reshape(-1)
+        V = rng.normal(size=U.size)
+        with FRSolver(cfg) as s:
+            Ud, out = torch.from_numpy(U).to(cuda), torch.empty(U.size, dtype=torch.float64, device=cuda)
+            s.pre_jv_eval(0.0, Ud, 1.0)
+            s.matmult(torch.from_numpy(V).to(cuda), out)
+        return out.cpu().numpy()
+    a, b = product(1e-30), product(2e-20)  # first order, complex: second-order terms at 4e-40
+    d = np.abs(a - b) / np.abs(b).max()
+    assert np.median(d) <= 64 * 2.0 ** -53
