@@ -354,7 +354,6 @@ int frsdg_create(const frsdg_config* cfg, frsdg_handle** out)
         a.Ly = cfg->box_length[1];
         a.ops = ops;
         a.bad = h->d_bad;
-        a.nd = 4 * n * n;
         a.exact_bc = cfg->jvp_exact_bc;
         a.tc = cfg->mixed_tc ? 1 : 0;
         for (int d = 0; d < 4; ++d)

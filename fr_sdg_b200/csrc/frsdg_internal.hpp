@@ -113,7 +113,6 @@ struct Fr2dArgs
     double h, inv_h, sigma;
     unsigned long long* bad;
     StageArgs st;
-    int    nd;         // DOFs per element, 4 n^2
     int    out_f32;    // residual written as float (FP32 instantiation)
     // row window (domain decomposition): the vectors hold Ny element rows starting at
     // global row row_base; rows [row_begin, row_end) are computed, the others are ghosts

@@ -8,7 +8,7 @@
 namespace frsdg
 {
 // Largest element block the preconditioner inverts (p <= 5 in 2D: 4 (p+1)^2 <= 144);
-// the FP64 block sits in one CTA's shared memory.
+// the block sits in one CTA's registers, 9 x 9 FP64 entries a thread at p = 5.
 constexpr int kMaxBlockDofs = 144;
 
 // What one launch over the elements' Jacobian blocks leaves (jac2d.cuh): the blocks

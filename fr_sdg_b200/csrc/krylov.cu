@@ -37,7 +37,8 @@ constexpr int kKryMaxBasis = 256;                           // Arnoldi vectors p
 static int64_t kry_blocks(int64_t n) { return (n + kKryChunk - 1) / kKryChunk; }
 
 // work layout (doubles): part[(kKryMaxBasis + 1) * B] | h1[kKryMaxBasis] | h2[kKryMaxBasis] |
-// scalars[4] (0: ||w||^2 before, 1: ||w||^2 after the first pass; 2, 3 unused)
+// scalars[4] (0: ||w||^2 before, 1: ||w||^2 after the first pass; 2 and 3 spare, as the size of
+// `work` is part of the interface)
 struct KryWork
 {
     double* part;

@@ -96,7 +96,8 @@ template <int N, int GEO, int VAR = 0, class S = double> struct Line2D
     }
     // Co-resident CTAs: what shared memory admits, at most 16 warps at n <= 4 and in the small
     // variant (128 registers), 15 at n = 5, 12 above (168 registers: at n = 6, 15 warps with
-    // narrower strides spill, 0.80 against 0.73 ms on the 1024^2 blast; nine warps are as fast);
+    // narrower strides spill, 0.80 against 0.73 ms on the 1024^2 blast; nine warps are as fast; n >= 7
+    // not swept, and the affine tuned tile spills 0.2 KB at n = 8 and 0.7 KB at n = 10);
     // FP32 16 (512^2 blast, p = 3, 4, 5: 0.134, 0.201, 0.217 ms with the face tiles, 0.059,
     // 0.094, 0.117 here; 12 to 24 warps within 8 %)
     static constexpr int CTAS_SM = int((227 * 1024) / (bytes + 1024));
@@ -982,19 +983,28 @@ cudaError_t launch_line_v(const Fr2dArgs& a, cudaStream_t st)
 // one tile's chain, which its face warps shorten (64^2 elements, affine / curved: p = 3 6.5 /
 // 7.4 -> 4.7 / 5.2 us, p = 4 8.1 / 8.6 -> 6.1 / 7.2, p = 5 8.4 / 10.0 -> 7.4 / 8.6); beyond one
 // residency the tuned tile does less halo work per element (96^2: p = 3 8.1 -> 7.4, p = 5
-// 12.9 -> 10.5 us).  Curved p = 5, whose tuned tile fills few warps, takes it at any size (256^2
-// vortex 0.143 -> 0.126 ms).
+// 12.9 -> 10.5 us).  Curved meshes, small / tuned at 48^2, 96^2, 200^2: p = 3 0.74, 0.77, 1.16; p = 4
+// 0.79, 1.00, 1.13; p = 6 0.84, 1.33, 1.42; p = 7 0.90, 1.28, 1.40; p = 8 1.06, 1.43, 1.46; p = 9 1.22,
+// 1.35, 1.49 (one residency ends at 69^2 up to n = 6, at 49^2 above, where p = 9 is on the wrong side
+// of it).  Curved p = 5, whose tuned tile fills few warps, takes the small variant at any size:
+// 0.81, 0.85, 0.85, and 0.87 at 256^2.
 template <class S, int N, int GAS, int RIEM, int GEO> cudaError_t launch_line(const Fr2dArgs& a, cudaStream_t st)
 {
     using L = Line2D<N, GEO, 2, S>;
-    const int64_t tiles = int64_t((a.Nx + L::TX - 1) / L::TX) * ((a.row_end - a.row_begin + L::TY - 1) / L::TY);
-    const bool small = tiles <= L::CTAS * kSMs || (GEO == GEO_CURVED && N == 6 && !L::F32);
-    if constexpr (!L::F32)
+    const bool post = !L::F32 && a.mode == MODE_STAGE && a.post;
+    auto launch = [&](auto var) -> cudaError_t {
+        constexpr int VAR = decltype(var)::value;
+        if constexpr (!L::F32)
+            if (post) return launch_line_v<S, N, GAS, RIEM, GEO, VAR, true>(a, st);
+        return launch_line_v<S, N, GAS, RIEM, GEO, VAR, false>(a, st);
+    };
+    if constexpr (GEO == GEO_CURVED && N == 6 && !L::F32) return launch(std::integral_constant<int, 2>{});
+    else
     {
-        if (a.mode == MODE_STAGE && a.post)
-            return small ? launch_line_v<S, N, GAS, RIEM, GEO, 2, true>(a, st) : launch_line_v<S, N, GAS, RIEM, GEO, 0, true>(a, st);
+        const int64_t tiles = int64_t((a.Nx + L::TX - 1) / L::TX) * ((a.row_end - a.row_begin + L::TY - 1) / L::TY);
+        if (tiles <= L::CTAS * kSMs) return launch(std::integral_constant<int, 2>{});
+        return launch(std::integral_constant<int, 0>{});
     }
-    return small ? launch_line_v<S, N, GAS, RIEM, GEO, 2, false>(a, st) : launch_line_v<S, N, GAS, RIEM, GEO, 0, false>(a, st);
 }
 
 } // namespace frsdg

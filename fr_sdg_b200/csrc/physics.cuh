@@ -328,8 +328,8 @@ __device__ __forceinline__ void riemann_rec(const S L[RF_N], const S R[RF_N], do
     Fs[3] = f3;
 }
 
-// The same face flux for real scalars, with the normal fluxes F.n of both sides: AXIS 0 an
-// x-face (n = (1, 0)), 1 a y-face (n = (0, 1)), 2 any normal.  HLLC's sampling
+// The same face flux for real scalars, with the normal fluxes F.n of both sides: AXIS 0 the
+// velocities in the face's frame (n = (1, 0)), 2 any normal.  HLLC's sampling
 // (riemann_solver.hpp:314-341) as one choice of side K and one of star state or F_K: the
 // outer states are F_L when s_L >= 0 and F_R when neither s_M nor s_R is non-negative, and
 // K is that side in both.
@@ -337,10 +337,10 @@ template <int RIEM, int AXIS, class S, class M>
 __device__ __forceinline__ void riemann_sides(const S L[RF_N], const S R[RF_N], S nx, S ny, S Fs[4], S FnL[4],
                                               S FnR[4], const M& m)
 {
-    const S unL = AXIS == 0 ? L[RF_U] : AXIS == 1 ? L[RF_V] : L[RF_U] * nx + L[RF_V] * ny;
-    const S utL = AXIS == 0 ? L[RF_V] : AXIS == 1 ? -L[RF_U] : -L[RF_U] * ny + L[RF_V] * nx;
-    const S unR = AXIS == 0 ? R[RF_U] : AXIS == 1 ? R[RF_V] : R[RF_U] * nx + R[RF_V] * ny;
-    const S utR = AXIS == 0 ? R[RF_V] : AXIS == 1 ? -R[RF_U] : -R[RF_U] * ny + R[RF_V] * nx;
+    const S unL = AXIS == 0 ? L[RF_U] : L[RF_U] * nx + L[RF_V] * ny;
+    const S utL = AXIS == 0 ? L[RF_V] : -L[RF_U] * ny + L[RF_V] * nx;
+    const S unR = AXIS == 0 ? R[RF_U] : R[RF_U] * nx + R[RF_V] * ny;
+    const S utR = AXIS == 0 ? R[RF_V] : -R[RF_U] * ny + R[RF_V] * nx;
     const S cL = L[RF_C], cR = R[RF_C], pL = L[RF_P], pR = R[RF_P];
     // fluxes in the frame (n, t)
     const S FL0 = L[RF_RHO] * unL, FR0 = R[RF_RHO] * unR;
@@ -384,8 +384,8 @@ __device__ __forceinline__ void riemann_sides(const S L[RF_N], const S R[RF_N], 
     }
     auto back = [&](const S v[4], S o[4]) {
         o[0] = v[0];
-        o[1] = AXIS == 0 ? v[1] : AXIS == 1 ? -v[2] : v[1] * nx - v[2] * ny;
-        o[2] = AXIS == 0 ? v[2] : AXIS == 1 ? v[1] : v[1] * ny + v[2] * nx;
+        o[1] = AXIS == 0 ? v[1] : v[1] * nx - v[2] * ny;
+        o[2] = AXIS == 0 ? v[2] : v[1] * ny + v[2] * nx;
         o[3] = v[3];
     };
     back(f, Fs);
