@@ -288,7 +288,8 @@ struct MathDeferred
     }
     __device__ __forceinline__ float sqrt(float x) const
     {
-        bad |= (__float_as_uint(x) >> 23) - 2u < 250u ? 0u : 1u;  // positive, 2^-125 <= x < 2^125
+        // positive, 2^-100 <= x < 2^125 (below, the correction's x - s^2 is subnormal)
+        bad |= (__float_as_uint(x) >> 23) - 27u < 225u ? 0u : 1u;
         float y;
         asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
         const float s = x * y;

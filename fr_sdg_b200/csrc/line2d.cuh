@@ -250,9 +250,9 @@ __device__ __forceinline__ void line_epilogue(const Fr2dArgs& a, const Ops& ops,
         __syncthreads();  // s_flag
     const PPView v{GAS == 0 ? FRSDG_GAS_IDEAL : FRSDG_GAS_VDW, a.gas, P.pp_eps, P.w, P.detJ};
     const double thr = v.eps0 * (1.0 + 1e-10);
+    bool clear = true;
     if (own)
     {
-        bool clear = true;
         unsigned bad = 0;
 #pragma unroll
         for (int l = 0; l < N; ++l)
@@ -266,28 +266,32 @@ __device__ __forceinline__ void line_epilogue(const Fr2dArgs& a, const Ops& ops,
                 clear = clear && u[0] > thr && pp_pressure_fast(v, u, MathDeferred{bad}) > thr;
             }
         }
-        if (!clear || bad) s_flag[e] = 1;
+        clear = clear && !bad;
+        if (!clear) s_flag[e] = 1;
     }
     if (!limit && !want_amax) return;
-    __syncthreads();  // flags and stores
     if (want_amax)
     {
+        // every node above the floor as it leaves the stage, in marked elements too (as the tiles
+        // of mixed stages: both forms of a batch then take the same steps); the limiter adds
+        // the marked elements' speeds after limiting
         double w = 0.0;
-        if (own && !s_flag[e])
+        if (own)
         {
 #pragma unroll 1
             for (int l = 0; l < N; ++l)
             {
-                const double2* o = reinterpret_cast<const double2*>(out + l * N * 4);
+                const double2* o = reinterpret_cast<const double2*>(out + l * N * 4);  // this thread's own stores
                 const double2 x = o[0], y = o[1];
                 const double u[4] = {x.x, x.y, y.x, y.y};
-                w = fmax(w, node_wave_speed_fast(v, u));
+                if (clear || (u[0] > thr && pp_pressure_fast(v, u) > thr)) w = fmax(w, node_wave_speed_fast(v, u));
             }
         }
         w = -pp_warp_min(-w);
         if ((tid & 31) == 0 && w > 0.0 && w < 1e300)
             atomicMax(&s_amax, static_cast<unsigned long long>(__double_as_longlong(w)));
     }
+    __syncthreads();  // flags and stores
     if (limit)
     {
         double* base = static_cast<double*>(a.out);

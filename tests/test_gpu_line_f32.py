@@ -12,7 +12,7 @@ from fr_sdg_b200.workloads import make_config
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("op,exponents", [(4, (-100, 0, 37)), (5, (-100, 0, 1, 38))])
+@pytest.mark.parametrize("op,exponents", [(4, (-125, -100, 0, 37, 123)), (5, (-125, -112, -101, -100, -99, 0, 1, 38, 123))])
 def test_fast_forms_equal_ieee(op, exponents, cuda):
     """Every mantissa (and either parity of the root's exponent): the fast FP32 reciprocal and root
     are the correctly rounded ones, so a redo with the IEEE operations leaves the same bits.  FP64
