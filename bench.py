@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -318,16 +319,18 @@ def batched_to_t_end(device, t_end: float = 0.25, max_steps: int = 4000) -> dict
         e = density_l2(cfg, Um, Ud)
         errs.append(e)
         rels.append(e / density_l2(cfg, Ud, torch.zeros_like(Ud)))
+    # instances whose mixed run ended non-finite stay in per_instance, out of the statistics
+    e_fin, r_fin = [e for e in errs if math.isfinite(e)], [r for r in rels if math.isfinite(r)]
     out.update({
         "t_end": t_end, "max_replays": max_steps,
         "scheme": "SSP-RK3, spectral filter + positivity limiter (floor 1e-6) on every stage, CFL 0.1 "
                   "(dt = CFL h / ((2p+1) max(|v|+c)) per instance, re-evaluated on the device after every step; "
                   "an instance whose step falls below 1e-3 of its first stops); the batch engine: one launch "
-                  "per order group and stage plus the limiter pass, the post-step in the last stage's "
-                  "epilogue, one CUDA graph per step of all instances, device clocks, autotuned tiles "
+                  "per order group and stage, the limiter in its epilogue (FP64) or as a pass (mixed), the "
+                  "post-step in the last stage's epilogue, one CUDA graph per step of all instances, device clocks, autotuned tiles "
                   "(the autotuner's first pass is inside the timed region)",
-        "mixed_vs_fp64_density_l2": {"max": max(errs), "median": statistics.median(errs),
-                                     "relative_max": max(rels), "relative_median": statistics.median(rels),
+        "mixed_vs_fp64_density_l2": {"max": max(e_fin), "median": statistics.median(e_fin),
+                                     "relative_max": max(r_fin), "relative_median": statistics.median(r_fin),
                                      "per_instance": [float(f"{e:.3e}") for e in errs]},
     })
     return out
@@ -699,9 +702,11 @@ def run_ours(args, ws, rank, local):
                     jvp_ms = rep(lambda: bs.matmult(Vb, Jb), 20)
                     bs.pc_setup(0.0, 10.0, B)
                     pcj_setup_ms = rep(lambda: bs.pc_setup(0.0, 10.0, B), 3)
+                    bs.pc_apply(Vb, Zb)  # the first launch loads the kernel
                     pcj_apply_ms = rep(lambda: bs.pc_apply(Vb, Zb), 20)
                     bs.pc_setup_gs(0.0, 10.0, B)
                     pcg_setup_ms = rep(lambda: bs.pc_setup_gs(0.0, 10.0, B), 3)
+                    bs.pc_apply(Vb, Zb)
                     pcg_apply_ms = rep(lambda: bs.pc_apply(Vb, Zb), 20)
                     nk = BackwardEulerNewtonKrylov(bs, restart=60, gmres_rtol=1e-6, max_gmres=600, newton_rtol=1e-8,
                                                    precondition="gs")

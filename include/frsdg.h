@@ -240,7 +240,8 @@ int frsdg_rk_stage_fused(frsdg_handle* h, double t, const double* Us, const doub
  * 72-95, 244).  The columns are assembled from the complex-step derivatives of the node
  * and face fluxes and equal single-seed products of frsdg_jvp up to rounding.  blocks:
  * nelem * nd * nd doubles (nd = 4 (p+1)^2), block e column-major:
- * blocks[(e*nd + col)*nd + row].  2D only. */
+ * blocks[(e*nd + col)*nd + row].  2D only.  Under a row window nelem counts the window's
+ * elements, and the blocks of its computed rows are written. */
 int frsdg_jac_blocks(frsdg_handle* h, double t, double sigma, const double* U,
                      double* blocks, void* stream);
 
