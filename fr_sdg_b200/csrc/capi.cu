@@ -156,6 +156,8 @@ int report_cuda(cudaError_t e, const char* what) { return cuda_fail(e, what); }
 // Element count and vector length of the vectors the entry points see.
 static int64_t local_nelem(const frsdg_handle* h) { return h->win_rows ? int64_t(h->Nx) * h->win_rows : h->nelem; }
 static int64_t local_ntot(const frsdg_handle* h) { return local_nelem(h) * h->ndofs; }
+// The longest vector of any row window: two ghost rows beside the whole mesh.
+static int64_t longest_ntot(const frsdg_handle* h) { return h->ntot + (h->cfg.dim == 2 ? int64_t(2) * h->Nx * h->ndofs : 0); }
 static void apply_window(const frsdg_handle* h, Fr2dArgs& a)
 {
     if (!h->win_rows) return;
@@ -530,7 +532,7 @@ int frsdg_create(const frsdg_config* cfg, frsdg_handle** out)
         for (int q = 0; q < n; ++q) s.w[q] = h->re.w[q];
         if (cfg->apply_weno && !cfg->apply_filter)
         {
-            cudaError_t e = cudaMalloc(&h->d_work, sizeof(double) * h->ntot);
+            cudaError_t e = cudaMalloc(&h->d_work, sizeof(double) * longest_ntot(h));
             if (e != cudaSuccess)
             {
                 free_handle(h);
@@ -1061,11 +1063,11 @@ int frsdg_rhs_host(frsdg_handle* h, double t, const double* U_host, double* rhs_
     cudaError_t e;
     if (!h->d_stage)
     {
-        e = cudaMalloc(&h->d_stage, sizeof(double) * 2 * h->ntot);
+        e = cudaMalloc(&h->d_stage, sizeof(double) * 2 * longest_ntot(h));
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(staging)");
     }
     double* dU = h->d_stage;
-    double* dR = h->d_stage + h->ntot;
+    double* dR = h->d_stage + longest_ntot(h);
     const int C = std::min(frsdg_handle::kHostChunks, h->Ny / 4);
     const bool chunked = h->cfg.dim == 2 && !h->win_rows && C >= 2;
     if (!chunked)

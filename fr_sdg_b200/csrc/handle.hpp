@@ -30,8 +30,8 @@ struct frsdg_handle
     double*      d_detJ = nullptr;   // positivity limiter on curved meshes: detJ per node
     frsdg::PPArgs       pp{};               // template of the positivity limiter's launch
     frsdg::PostArgs*    d_post = nullptr;   // 2D: operands of the fused stage epilogue
-    double*      d_work = nullptr;   // post-step source copy (WENO)
-    double*      d_stage = nullptr;  // host-buffer staging (2 * ntot), allocated on first use
+    double*      d_work = nullptr;   // post-step source copy (WENO), as long as any row window
+    double*      d_stage = nullptr;  // host-buffer staging (two vectors of any row window), allocated on first use
     unsigned long long* d_bad = nullptr;
     // preconditioner, allocated by the first set-up: the FP32 inverses of the element-diagonal
     // Jacobian blocks, the neighbours' nonzeros (Gauss-Seidel; jac2d.cuh), the pivot flag
